@@ -44,10 +44,10 @@ static const int MONOLIS_B200_PRM_I_REFRESH_PERIOD = 41; /* mixed precision: FP6
 static const int MONOLIS_B200_PRM_I_WIDE_SLICES_FP64 = 42; /* out: 32-row slices that keep 32-bit column ids (the
                                                               others store 16-bit differences to a base per slot) */
 static const int MONOLIS_B200_PRM_I_WIDE_SLICES_FP32 = 43; /* out: same for the 64-row slices of the FP32 layout */
-static const int MONOLIS_B200_PRM_I_WAIT_LIMIT     = 44; /* many right-hand sides: polls after which a grid-barrier
+static const int MONOLIS_B200_PRM_I_WAIT_LIMIT     = 44; /* many right-hand sides and one-kernel solves: polls after which a grid-barrier
                                                             wait gives up and the solve returns MONOLIS_B200_TIMEOUT
                                                             (0: 4,194,304, seconds) */
-static const int MONOLIS_B200_PRM_I_WAIT_DELAY_US  = 45; /* testing that bound: block 0 of the many-right-hand-side
+static const int MONOLIS_B200_PRM_I_WAIT_DELAY_US  = 45; /* testing that bound: block 0 of the
                                                             kernel reaches its first barrier this many microseconds
                                                             late (0: off; at most 1,000,000) */
 static const int MONOLIS_B200_PRM_I_UNIFORM_SLICES_FP64 = 46; /* out: 32-row slices whose block columns are the

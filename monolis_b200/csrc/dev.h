@@ -88,6 +88,8 @@ struct SellMatrix {
   int* d_cbase2 = nullptr;
   long long wide64 = 0, wide32 = 0;  // slices that keep 32-bit column ids
   long long uniform64 = 0, uniform32 = 0;  // slices whose columns are the slot bases + lane (bit 1 of slc)
+  int below = 0, above = 0;  // band: the columns of row i lie in [i - below, i + above]
+  int wmax = 0;              // longest row
   double bytes64 = 0, bytes32 = 0;   // HBM bytes of one SpMV in each layout
   // unroll depth (slots in flight per thread) picked by the autotuner
   int u64 = 2, u32 = 2;
@@ -99,11 +101,18 @@ struct SellMatrix {
   // upload staging (kept between solves)
   int* d_item = nullptr;          // CSR items as uploaded (1-based)
   double* d_csrval = nullptr;
+  int* d_perm = nullptr;          // a transpose: CSR position (1-based) of each of its blocks
+  size_t cap_perm = 0;
   size_t cap_rowptr = 0, cap_slptr = 0, cap_col = 0, cap_val64 = 0, cap_val32 = 0;
   size_t cap_alu64 = 0, cap_alu32 = 0, cap_item = 0, cap_csrval = 0, cap_slptr2 = 0, cap_col2 = 0;
   size_t cap_slc = 0, cap_col16 = 0, cap_cbase = 0, cap_slc2 = 0, cap_col16p = 0, cap_cbase2 = 0;
   bool have_val32 = false, have_alu = false, have_alu32 = false;
 };
+
+// Stream-ordered allocation from the library's own pool (solve.cu: work_pool),
+// freed with cudaFreeAsync: the memory stays mapped in the pool, where the
+// default pool gives it back to the driver at every synchronisation.
+cudaError_t pool_alloc(void** p, size_t bytes, cudaStream_t s);
 
 struct Scratch {
   double* partials = nullptr;     // (65536 + 256) * 4 doubles: block and group partial sums
@@ -120,10 +129,16 @@ int sell_build(SellMatrix& m, const int* h_index, const int* h_item, const doubl
                int N, int ndof, cudaStream_t s, double* t_h2d);
 // Slices and FP64 values from the device CSR (d_rowptr, d_item, d_csrval).
 int sell_layout(SellMatrix& m, cudaStream_t s);
+// The device CSR values have changed, the pattern has not: FP64 values of the
+// layout again (the FP32 copy and the DIAG factors follow on demand).
+int sell_refill(SellMatrix& m, cudaStream_t s);
+void sell_values_changed(SellMatrix& m);  // drops the FP32 copy and the DIAG factors
 // A^T from A's device CSR and the host CSC arrays of the pattern (offsets,
 // 1-based rows, 1-based CSR positions; monolis_get_CSC_format).
 int sell_build_transpose(SellMatrix& at, const SellMatrix& a, const int* h_csc_index, const int* h_csc_item,
                          const int* h_csc_perm, cudaStream_t s);
+// A^T's values again after A's changed, the pattern being the one at was built for.
+int sell_refill_transpose(SellMatrix& at, const SellMatrix& a, cudaStream_t s);
 int sell_make_fp32(SellMatrix& m, cudaStream_t s);
 // Times the SpMV unroll variants on the matrix and keeps the fastest (u64 / u32).
 int sell_autotune(SellMatrix& m, bool fp32, cudaStream_t s);
@@ -204,6 +219,8 @@ struct SolveParams {
   int timers;        // time every kernel with CUDA events (no graph)
   const ShardPlan* shard = nullptr;  // multi-rank solve (FP64 CG); x holds np_rows block rows (ghosts last)
   int np_rows = 0;
+  unsigned long long wait_limit = 0;  // one-kernel solves: polls before a grid-wide wait gives up (0: the default, seconds)
+  unsigned int delay_ns = 0;          // testing that bound: block 0 starts that much later
 };
 struct SolveResult {
   int iter = 0, status = 0, n_refine = 0;
@@ -217,7 +234,17 @@ struct SolveResult {
 int solve_device(SellMatrix& m, Scratch& sc, const SolveParams& p, const double* d_b, double* d_x,
                  SolveResult& res, double* h_hist, cudaStream_t s);
 
-// ---- device assembly (assemble.cu): values of m's device CSR (d_csrval) ----
+// ---- one-kernel solves (persist.cu) ----
+// persist_applies: the rule by which solve_device takes them. work:
+// persist_work_bytes() of device memory. The verdict is left in *st (not done
+// if a wait gave up).
+bool persist_applies(const SellMatrix& m, const SolveParams& p);
+size_t persist_work_bytes(const SellMatrix& m, const SolveParams& p);
+int persist_solve(const SellMatrix& m, const SolveParams& p, const double* b, double* x, void* work, SolverState* st,
+                  double* hist, cudaStream_t s);
+
+// ---- device assembly (assemble.cu): values of m's device CSR (d_csrval) and FP64 layout ----
+int device_clear_values(SellMatrix& m, cudaStream_t s);
 int device_add_elements(SellMatrix& m, int NP, int n_elem, int n_base, const int* d_elem, const double* d_val,
                         long long val_stride, const double* d_scale, cudaStream_t s);
 // node/dof/val: host lists of n_bc conditions, applied as if in order; d_b device RHS

@@ -1,5 +1,6 @@
 // sell.cu -- device matrix build (CSR upload -> sliced ELL), DIAG factor
 // setup, and the standalone SpMV / inner product / DIAG apply kernels.
+#include <algorithm>
 #include <cstdio>
 #include <cstring>
 #include <vector>
@@ -72,8 +73,9 @@ __global__ void sell2_fill_kernel(const int* __restrict__ rowptr, const int* __r
   }
 }
 
-// One warp per slice: lane l copies row (32s + l) into the slot-major layout.
-template <int B>
+// One warp per slice: lane l copies row (32s + l) into the slot-major layout
+// (kCols: column ids too; without, the values of an unchanged pattern only).
+template <int B, bool kCols>
 __global__ void sell_fill_kernel(const int* __restrict__ rowptr, const int* __restrict__ item,
                                  const double* __restrict__ csrval, const long long* __restrict__ slptr,
                                  int N, int nslices, int* __restrict__ col, double* __restrict__ val) {
@@ -89,10 +91,10 @@ __global__ void sell_fill_kernel(const int* __restrict__ rowptr, const int* __re
   for (int k = 0; k < w; k++) {
     const long long slot = base + (long long)k * kSlice;
     if (k < len) {
-      col[slot + lane] = item[j0 + k] - 1;
+      if (kCols) col[slot + lane] = item[j0 + k] - 1;
 #pragma unroll
       for (int e = 0; e < B2; e++) val[(slot * B2) + (long long)e * kSlice + lane] = csrval[(j0 + k) * B2 + e];
-    } else {
+    } else if (kCols) {
       col[slot + lane] = row < N ? row : 0;
 #pragma unroll
       for (int e = 0; e < B2; e++) val[(slot * B2) + (long long)e * kSlice + lane] = 0.0;
@@ -118,7 +120,7 @@ __global__ void sell_fill_kernel(const int* __restrict__ rowptr, const int* __re
 // position, and the difference stream is not read at all.
 // stats: [0] wide slices, [1] real blocks in wide slices, [2] slot positions
 // of compressed slices (uniform ones included), [3] real blocks in uniform
-// slices, [4] uniform slices.
+// slices, [4] uniform slices, [5] max(row - column), [6] max(column - row).
 template <int P>
 __global__ void col_compact_kernel(const int* __restrict__ rowptr, const long long* __restrict__ slptr, int N,
                                    int nslices, const int* __restrict__ col, short* __restrict__ col16,
@@ -138,6 +140,7 @@ __global__ void col_compact_kernel(const int* __restrict__ rowptr, const long lo
   }
   bool fit = true, uni = true;
   unsigned long long nreal = 0;
+  int lo = 0, hi = 0;  // band of the slice's rows
   for (int k = 0; k < w; k++) {
     const long long slot = base + (long long)k * H;
     int c[P];
@@ -155,6 +158,8 @@ __global__ void col_compact_kernel(const int* __restrict__ rowptr, const long lo
     emin = __reduce_min_sync(0xffffffffu, emin);
     emax = __reduce_max_sync(0xffffffffu, emax);
     const long long c0 = (long long)emin + (((long long)emax - emin) >> 1);
+    lo = max(lo, (int)(warp * H - emin));
+    hi = max(hi, (int)(emax - warp * H));
 #pragma unroll
     for (int h = 0; h < P; h++) {
       const long long pos = (long long)P * lane + h;
@@ -178,6 +183,8 @@ __global__ void col_compact_kernel(const int* __restrict__ rowptr, const long lo
   for (int o = 16; o > 0; o >>= 1) nreal += __shfl_xor_sync(0xffffffffu, nreal, o);
   if (lane == 0) {
     slc[warp] = base | (fit ? 0 : 1) | (uni ? 2 : 0);
+    atomicMax(&stats[5], (unsigned long long)lo);
+    atomicMax(&stats[6], (unsigned long long)hi);
     if (!fit) {
       atomicAdd(&stats[0], 1ULL);
       atomicAdd(&stats[1], nreal);
@@ -304,25 +311,28 @@ __global__ void diag_apply_kernel(const double* __restrict__ alu, int N, const d
 template <int P>
 int compact_columns(const SellMatrix& m, const long long* d_slptr, int nslices, long long padded,
                     const int* d_col, short** col16, size_t& cap16, int** cbase, size_t& capb, long long** slc,
-                    size_t& capslc, long long& wide, long long& uniform, double& col_bytes, cudaStream_t s) {
+                    size_t& capslc, long long& wide, long long& uniform, double& col_bytes, cudaStream_t s,
+                    int* below = nullptr, int* above = nullptr) {
   MB_CUDA_OK(grow(col16, cap16, (size_t)padded + 2));
   MB_CUDA_OK(grow(cbase, capb, (size_t)(padded / (32 * P)) + 1));
   MB_CUDA_OK(grow(slc, capslc, (size_t)nslices + 1));
   unsigned long long* d_stats = nullptr;
-  MB_CUDA_OK(cudaMallocAsync((void**)&d_stats, 5 * sizeof(unsigned long long), s));
-  MB_CUDA_OK(cudaMemsetAsync(d_stats, 0, 5 * sizeof(unsigned long long), s));
+  MB_CUDA_OK(pool_alloc((void**)&d_stats, 7 * sizeof(unsigned long long), s));
+  MB_CUDA_OK(cudaMemsetAsync(d_stats, 0, 7 * sizeof(unsigned long long), s));
   if (nslices > 0) {
     const long long threads = (long long)nslices * 32;
     col_compact_kernel<P><<<(unsigned)((threads + 255) / 256), 256, 0, s>>>(m.d_rowptr, d_slptr, m.N, nslices, d_col,
                                                                           *col16, *cbase, *slc, d_stats);
   }
-  unsigned long long st[5] = {0, 0, 0, 0, 0};
+  unsigned long long st[7] = {0, 0, 0, 0, 0, 0, 0};
   MB_CUDA_OK(cudaGetLastError());
   MB_CUDA_OK(cudaMemcpyAsync(st, d_stats, sizeof(st), cudaMemcpyDeviceToHost, s));
   MB_CUDA_OK(cudaStreamSynchronize(s));
   cudaFreeAsync(d_stats, s);
   wide = (long long)st[0];
   uniform = (long long)st[4];
+  if (below) *below = (int)st[5];
+  if (above) *above = (int)st[6];
   col_bytes = 2.0 * (double)(m.nz - (long long)st[1] - (long long)st[3]) + 4.0 * (double)st[1] + 4.0 * (double)st[2];
   return kOk;
 }
@@ -364,18 +374,22 @@ int sell_layout(SellMatrix& m, cudaStream_t s) {
   const int B2 = ndof * ndof;
   const int nslices = (N + kSlice - 1) / kSlice;
   m.nslices = nslices;
-  m.have_val32 = m.have_alu = m.have_alu32 = false;
+  sell_values_changed(m);
   MB_CUDA_OK(grow(&m.d_slptr, m.cap_slptr, (size_t)nslices + 1));
   // slice widths -> prefix on the host (nslices = N/32 values) -> slice pointers
   long long* d_w = nullptr;
-  MB_CUDA_OK(cudaMallocAsync((void**)&d_w, sizeof(long long) * nslices, s));
+  MB_CUDA_OK(pool_alloc((void**)&d_w, sizeof(long long) * nslices, s));
   slice_width_kernel<<<(nslices + 255) / 256, 256, 0, s>>>(m.d_rowptr, N, nslices, kSlice, d_w);
   std::vector<long long> w(nslices), ptr(nslices + 1);
   MB_CUDA_OK(cudaMemcpyAsync(w.data(), d_w, sizeof(long long) * nslices, cudaMemcpyDeviceToHost, s));
   MB_CUDA_OK(cudaStreamSynchronize(s));
   cudaFreeAsync(d_w, s);
   ptr[0] = 0;
-  for (int i = 0; i < nslices; i++) ptr[i + 1] = ptr[i] + w[i];
+  m.wmax = 0;
+  for (int i = 0; i < nslices; i++) {
+    ptr[i + 1] = ptr[i] + w[i];
+    m.wmax = std::max(m.wmax, (int)(w[i] / kSlice));
+  }
   m.padded = ptr[nslices];
   MB_CUDA_OK(cudaMemcpyAsync(m.d_slptr, ptr.data(), sizeof(long long) * (nslices + 1), cudaMemcpyHostToDevice, s));
   MB_CUDA_OK(grow(&m.d_col, m.cap_col, (size_t)m.padded));
@@ -384,7 +398,7 @@ int sell_layout(SellMatrix& m, cudaStream_t s) {
   const int blocks = (int)(((long long)nslices * 32 + threads - 1) / threads);
   int rc = dispatch_ndof(ndof, [&](auto Bc) {
     constexpr int B = decltype(Bc)::value;
-    sell_fill_kernel<B><<<blocks, threads, 0, s>>>(m.d_rowptr, m.d_item, m.d_csrval, m.d_slptr, N, nslices, m.d_col,
+    sell_fill_kernel<B, true><<<blocks, threads, 0, s>>>(m.d_rowptr, m.d_item, m.d_csrval, m.d_slptr, N, nslices, m.d_col,
                                                    m.d_val64);
     return kOk;
   });
@@ -392,11 +406,29 @@ int sell_layout(SellMatrix& m, cudaStream_t s) {
   MB_CUDA_OK(cudaGetLastError());
   double col_bytes = 0;
   rc = compact_columns<1>(m, m.d_slptr, nslices, m.padded, m.d_col, &m.d_col16, m.cap_col16, &m.d_cbase, m.cap_cbase,
-                          &m.d_slc, m.cap_slc, m.wide64, m.uniform64, col_bytes, s);
+                          &m.d_slc, m.cap_slc, m.wide64, m.uniform64, col_bytes, s, &m.below, &m.above);
   if (rc) return rc;
   // values, column ids, row offsets, slice offsets, x once and y
   m.bytes64 = (double)m.nz * B2 * 8 + col_bytes + 4.0 * (N + 1) + 8.0 * nslices + 2.0 * N * ndof * 8;
   return sell_autotune(m, false, s);
+}
+
+void sell_values_changed(SellMatrix& m) { m.have_val32 = m.have_alu = m.have_alu32 = false; }
+
+// The FP64 values again from the device CSR values; slices and columns stay
+// (padded slots keep their zeros).
+int sell_refill(SellMatrix& m, cudaStream_t s) {
+  const unsigned blocks = (unsigned)(((long long)m.nslices * 32 + 255) / 256);
+  int rc = dispatch_ndof(m.ndof, [&](auto Bc) {
+    constexpr int B = decltype(Bc)::value;
+    sell_fill_kernel<B, false><<<blocks, 256, 0, s>>>(m.d_rowptr, m.d_item, m.d_csrval, m.d_slptr, m.N, m.nslices,
+                                                      m.d_col, m.d_val64);
+    return kOk;
+  });
+  if (rc) return rc;
+  MB_CUDA_OK(cudaGetLastError());
+  sell_values_changed(m);
+  return kOk;
 }
 
 int sell_make_fp32(SellMatrix& m, cudaStream_t s) {
@@ -404,7 +436,7 @@ int sell_make_fp32(SellMatrix& m, cudaStream_t s) {
   const int N = m.N, B2 = m.ndof * m.ndof;
   const int ns = (N + 63) / 64;
   long long* d_w = nullptr;
-  MB_CUDA_OK(cudaMallocAsync((void**)&d_w, sizeof(long long) * ns, s));
+  MB_CUDA_OK(pool_alloc((void**)&d_w, sizeof(long long) * ns, s));
   slice_width_kernel<<<(ns + 255) / 256, 256, 0, s>>>(m.d_rowptr, N, ns, 64, d_w);
   std::vector<long long> w(ns), ptr(ns + 1);
   MB_CUDA_OK(cudaMemcpyAsync(w.data(), d_w, sizeof(long long) * ns, cudaMemcpyDeviceToHost, s));
@@ -481,6 +513,7 @@ void sell_free(SellMatrix& m) {
   cudaFree(m.d_slc2);
   cudaFree(m.d_col16p);
   cudaFree(m.d_cbase2);
+  cudaFree(m.d_perm);
   m = SellMatrix();
 }
 
@@ -540,8 +573,8 @@ int sell_autotune(SellMatrix& m, bool fp32, cudaStream_t s) {
   const size_t n = (size_t)m.N * m.ndof;
   const size_t bytes = n * (fp32 ? sizeof(float) : sizeof(double));
   void *x = nullptr, *y = nullptr;
-  MB_CUDA_OK(cudaMallocAsync(&x, bytes + 16, s));
-  MB_CUDA_OK(cudaMallocAsync(&y, bytes + 16, s));
+  MB_CUDA_OK(pool_alloc(&x, bytes + 16, s));
+  MB_CUDA_OK(pool_alloc(&y, bytes + 16, s));
   MB_CUDA_OK(cudaMemsetAsync(x, 0, bytes, s));
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);

@@ -36,6 +36,7 @@
 #include <unordered_map>
 #include <vector>
 
+#include "krylov.cuh"
 #include "spmv.cuh"
 
 namespace mb {
@@ -102,55 +103,9 @@ __device__ __forceinline__ void for_rows(const RowSet& rs, int N, F&& body) {
 }
 
 // ---------------------------------------------------------------------------
-// Scalar updates run by the last block of a grid reduction.
+// Scalar updates run by the last block of a grid reduction (fin_cg, fin_bicg
+// and the FP32-refined ones: krylov.cuh).
 // ---------------------------------------------------------------------------
-__device__ void record(SolverState* st, double* hist, double resid) {
-  st->resid = resid;
-  if (hist) hist[st->iter] = resid;
-}
-
-// end of CG iteration `iter` (or the initial residual when iter == 0):
-// rr = <r,r>, rz = <r,z> (= rho of the next iteration).
-__device__ void fin_cg(SolverState* st, double rr, double rz, double* hist) {
-  if (st->iter == 0) {
-    st->B2 = rr;
-    if (rr == 0.0) { st->done = 1; st->status = kZeroRhs; return; }
-    st->rho = rz;
-    st->iter = 1;
-    return;
-  }
-  const double resid = sqrt(rr / st->B2);  // src/linalg/mat_converge.f90:120
-  record(st, hist, resid);
-  if (resid < st->tol) { st->done = 1; st->status = kOk; return; }
-  if (!isfinite(resid)) { st->done = 1; st->status = kNonFinite; return; }
-  if (st->iter >= st->max_iter) { st->done = 1; st->status = kMaxIter; return; }
-  st->rho1 = st->rho;
-  st->rho = rz;
-  st->beta = st->rho / st->rho1;  // src/iterative/CG.f90:79
-  st->iter += 1;
-}
-
-// end of BiCGSTAB iteration: rr = <R,R>, rrt = <R,RT> (= rho of the next one)
-__device__ void fin_bicg(SolverState* st, double rr, double rrt, double* hist) {
-  if (st->iter == 0) {
-    st->B2 = rr;
-    if (rr == 0.0) { st->done = 1; st->status = kZeroRhs; return; }
-    st->rho = rrt;
-    st->iter = 1;
-    return;
-  }
-  const double resid = sqrt(rr / st->B2);
-  record(st, hist, resid);
-  if (resid < st->tol) { st->done = 1; st->status = kOk; return; }
-  if (!isfinite(resid)) { st->done = 1; st->status = kNonFinite; return; }
-  if (st->iter >= st->max_iter) { st->done = 1; st->status = kMaxIter; return; }
-  st->rho1 = st->rho;
-  st->rho = rrt;
-  if (rrt == 0.0) { st->done = 1; st->status = kBreakdown; return; }
-  st->beta = (st->rho / st->rho1) * (st->alpha / st->omega);  // src/iterative/BiCGSTAB.f90:96
-  st->iter += 1;
-}
-
 // PipeCG (src/iterative/PipeCG.f90:93-149). Convergence check of an
 // iteration (or the initial residual when iter == 0): rr = <R,R>.
 __device__ void fin_pipe_check(SolverState* st, double rr, double* hist) {
@@ -833,8 +788,6 @@ __global__ void __launch_bounds__(kThreads, SpmvMinBlocks<B>::value)
 // n_ghost entries after the owned ones get the X update too (the FP32
 // correction of the multi-rank refined solve, kept with the owners'
 // arithmetic; PT and ST hold their ghost entries after the halo updates).
-__device__ void fin_mixed_bicg(SolverState* st, double rr, double rrt, double* hist);
-
 template <int B, class T, bool Mixed = false>
 __global__ void __launch_bounds__(kThreads)
     bicg_xr_kernel(int N, T* __restrict__ x, const T* __restrict__ pt, const T* __restrict__ stv,
@@ -929,45 +882,7 @@ __global__ void shard_bicg_kernel(SolverState* st, double* hist) {
 // Convergence is decided only on that FP64 residual. The fold x += y, y = 0
 // is done by the next p update (or after the loop).
 // ---------------------------------------------------------------------------
-__device__ void fin_mixed_inner(SolverState* st, double rr, double rz, double* hist) {
-  const double rn = sqrt(rr);
-  const double resid = sqrt(rr / st->B2);
-  record(st, hist, resid);
-  st->rho1 = st->rho;
-  if (!isfinite(resid)) { st->done = 1; st->status = kNonFinite; return; }
-  if (rn > st->rmax) st->rmax = rn;
-  if (rn < st->delta * st->rmax || resid < st->tol || st->iter >= st->max_iter ||
-      (st->period > 0 && st->iter - st->last_refresh >= st->period)) {
-    st->refresh = 1;  // the refresh kernel of this iteration finishes it
-    return;
-  }
-  st->rho = rz;
-  st->beta = st->rho / st->rho1;
-  st->iter += 1;
-}
-
-// Mixed precision BiCGSTAB: the same scheme on src/iterative/BiCGSTAB.f90's
-// recurrences. X + Y is the solution (Y accumulates alpha*PT + omega*ST in
-// FP32); a refresh recomputes R = B - A (X + Y) in FP64 and continues with
-// rho = <R,RT> of that residual, the shadow residual RT and P, V unchanged
-// (the reference's own true-residual replacement, made adaptive).
-__device__ void fin_mixed_bicg(SolverState* st, double rr, double rrt, double* hist) {
-  const double rn = sqrt(rr);
-  const double resid = sqrt(rr / st->B2);
-  record(st, hist, resid);
-  st->rho1 = st->rho;
-  if (!isfinite(resid)) { st->done = 1; st->status = kNonFinite; return; }
-  if (rn > st->rmax) st->rmax = rn;
-  if (rn < st->delta * st->rmax || resid < st->tol || st->iter >= st->max_iter ||
-      (st->period > 0 && st->iter - st->last_refresh >= st->period)) {
-    st->refresh = 1;
-    return;
-  }
-  st->rho = rrt;
-  if (rrt == 0.0) { st->done = 1; st->status = kBreakdown; return; }
-  st->beta = (st->rho / st->rho1) * (st->alpha / st->omega);
-  st->iter += 1;
-}
+// Scalar steps: fin_mixed_inner, fin_mixed_bicg (krylov.cuh).
 
 // V = A PT (FP32 paired layout); c2 = <RT,V>; alpha = rho/c2.
 template <int B, int U>
@@ -1235,38 +1150,6 @@ __global__ void __launch_bounds__(kThreads)
   });
 }
 
-// End of a refresh (or of the initial residual when iter == 0): rr = <r64,r64>,
-// rz = <r,z> (CG) or <r,rt> (BiCGSTAB).
-template <bool Bicg>
-__device__ void fin_mixed_refresh(SolverState* st, double rr, double rz, double* hist) {
-  if (st->iter == 0) {
-    st->B2 = rr;
-    if (rr == 0.0) { st->done = 1; st->status = kZeroRhs; return; }
-    st->rmax = sqrt(rr);
-    st->rho = rz;
-    st->iter = 1;
-    return;
-  }
-  const double resid = sqrt(rr / st->B2);
-  record(st, hist, resid);
-  st->refresh = 0;
-  st->fold = 1;
-  st->n_refine += 1;
-  st->last_refresh = st->iter;
-  if (resid < st->tol) { st->done = 1; st->status = kOk; return; }
-  if (!isfinite(resid)) { st->done = 1; st->status = kNonFinite; return; }
-  if (st->iter >= st->max_iter) { st->done = 1; st->status = kMaxIter; return; }
-  st->rmax = sqrt(rr);
-  st->rho = rz;
-  if (Bicg) {
-    if (rz == 0.0) { st->done = 1; st->status = kBreakdown; return; }
-    st->beta = (st->rho / st->rho1) * (st->alpha / st->omega);
-  } else {
-    st->beta = st->rho / st->rho1;
-  }
-  st->iter += 1;
-}
-
 // Multi-rank FP32-refined CG: the scalar steps with the all-reduced sums in red[].
 __global__ void shard_mixed_alpha_kernel(SolverState* st) {
   if (st->done) return;
@@ -1306,7 +1189,9 @@ __global__ void __launch_bounds__(kThreads, SpmvMinBlocks<B>::value)
                          SolverState* st, double* hist, float* __restrict__ rt = nullptr) {
   if (st->done || !(st->iter == 0 || st->refresh)) return;
   const bool init = st->iter == 0;
-  PlainAcc<2> v;
+  // CG: double-double, so the residual that decides convergence does not depend
+  // on the grouping of the sum (the one-kernel solve groups it otherwise)
+  std::conditional_t<Bicg, PlainAcc<2>, DDAcc<2>> v;
   const XPlusY xy{x, y};
   for (int row = blockIdx.x * blockDim.x + threadIdx.x; row < A.N; row += gridDim.x * blockDim.x) {
     // (A (x + y))[row] in FP64, blocks in CSR order, U slots in flight
@@ -1317,7 +1202,7 @@ __global__ void __launch_bounds__(kThreads, SpmvMinBlocks<B>::value)
     for (int c = 0; c < B; c++) {
       const long long i = (long long)row * B + c;
       const double rv = b[i] - ax[c];
-      v.s[0] += rv * rv;
+      v.add(0, rv, rv);
       t[c] = (float)rv;
       r[i] = t[c];
       w[c] = t[c];
@@ -1409,9 +1294,7 @@ struct Vecs {
   T* get(long long n) {
     const size_t bytes = (sizeof(T) * (size_t)(n > 0 ? n : 1) + 16 + 255) / 256 * 256;
     void* p = nullptr;
-    cudaMemPool_t pool = work_pool();
-    if ((pool ? cudaMallocFromPoolAsync(&p, bytes, pool, s) : cudaMallocAsync(&p, bytes, s)) != cudaSuccess)
-      return nullptr;
+    if (pool_alloc(&p, bytes, s) != cudaSuccess) return nullptr;
     extra.push_back(p);
     return static_cast<T*>(p);
   }
@@ -1436,6 +1319,11 @@ int largest_divisor_at_most(int v, int cap) {
 }
 
 }  // namespace
+
+cudaError_t pool_alloc(void** p, size_t bytes, cudaStream_t s) {
+  cudaMemPool_t pool = work_pool();
+  return pool ? cudaMallocFromPoolAsync(p, bytes, pool, s) : cudaMallocAsync(p, bytes, s);
+}
 
 int solve_device(SellMatrix& m, Scratch& sc, const SolveParams& p, const double* d_b, double* d_x,
                  SolveResult& res, double* h_hist, cudaStream_t s) {
@@ -1505,7 +1393,8 @@ int solve_device(SellMatrix& m, Scratch& sc, const SolveParams& p, const double*
   Plan plan;
   auto t0 = std::chrono::steady_clock::now();
 
-  rc = dispatch_ndof(nd, [&](auto Bc) -> int {
+  const bool one_kernel = persist_applies(m, p);
+  if (!one_kernel) rc = dispatch_ndof(nd, [&](auto Bc) -> int {
    constexpr int B = decltype(Bc)::value;
    return dispatch_u(p.precision == 0 ? m.u64 : m.u32, [&](auto Uc) -> int {
     constexpr int U = eff_u(B, decltype(Uc)::value);
@@ -2058,6 +1947,18 @@ int solve_device(SellMatrix& m, Scratch& sc, const SolveParams& p, const double*
     out = sc.h_st[0];
     return e;
   };
+
+  if (one_kernel) {
+    void* work = vec.get<char>((long long)persist_work_bytes(m, p));
+    if (!work) return kCudaError;
+    rc = persist_solve(m, p, d_b, d_x, work, sc.st, sc.hist, s);
+    if (rc) return rc;
+    SolverState fin{};
+    const cudaError_t e = read_state(fin);
+    if (e != cudaSuccess) return report_cuda(e, "one-kernel solve", __FILE__, __LINE__);
+    res.t_loop = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
+    return finish(fin);
+  }
 
   res.kernel_time.assign(plan.kernels, 0.0);
   SolverState cur{};

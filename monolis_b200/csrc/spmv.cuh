@@ -19,6 +19,26 @@ __device__ __forceinline__ T ldx(const T* p) {
   else return __ldg(p);
 }
 
+// Cache policy of the matrix stream: kStreamOnce reads with the evict-first
+// hint (a matrix larger than L2: keep the vectors resident instead),
+// kStreamKeep leaves it in L2 but not in L1 (solvers that re-read a matrix
+// that fits in L2 every iteration).
+enum StreamPolicy { kStreamOnce = 0, kStreamKeep = 1 };
+template <int P>
+__device__ __forceinline__ double ld_mat(const double* p) {
+  if constexpr (P == kStreamOnce) return __ldcs(p);
+  double v;
+  asm("ld.global.nc.L1::no_allocate.f64 %0, [%1];" : "=d"(v) : "l"(p));
+  return v;
+}
+template <int P>
+__device__ __forceinline__ float2 ld_mat(const float2* p) {
+  if constexpr (P == kStreamOnce) return __ldcs(p);
+  float2 v;
+  asm("ld.global.nc.L1::no_allocate.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p));
+  return v;
+}
+
 template <class V>
 struct SellView {
   const int* __restrict__ rowptr;
@@ -65,7 +85,7 @@ __device__ __forceinline__ void load_cols(bool wide, bool uniform, const int* __
 // each thread keeps U*(B*B + 1) independent loads in flight.
 // xf(i) gives entry i = column*B + l of the multiplied vector. kCols16 =
 // false reads the 32-bit column ids of every slice.
-template <int B, int U, class V, class T, bool kCols16 = true, class XF>
+template <int B, int U, class V, class T, bool kCols16 = true, int P = kStreamOnce, class XF>
 __device__ __forceinline__ void sell_row_f(const SellView<V>& A, const XF xf, int row, T (&y)[B]) {
   constexpr int B2 = B * B;
   const int lane = row & (kSlice - 1);
@@ -88,7 +108,7 @@ __device__ __forceinline__ void sell_row_f(const SellView<V>& A, const XF xf, in
 #pragma unroll
     for (int u = 0; u < U; u++)
 #pragma unroll
-      for (int e = 0; e < B2; e++) a[u][e] = ld_stream(v + ((long long)(k + u) * B2 + e) * kSlice);
+      for (int e = 0; e < B2; e++) a[u][e] = ld_mat<P>(v + ((long long)(k + u) * B2 + e) * kSlice);
 #pragma unroll
     for (int u = 0; u < U; u++) {
       T xs[B];
@@ -110,7 +130,7 @@ __device__ __forceinline__ void sell_row_f(const SellView<V>& A, const XF xf, in
 #pragma unroll
     for (int u = 0; u < U; u++)
 #pragma unroll
-      for (int e = 0; e < B2; e++) a[u][e] = u < rem ? ld_stream(v + ((long long)(k + u) * B2 + e) * kSlice) : V(0);
+      for (int e = 0; e < B2; e++) a[u][e] = u < rem ? ld_mat<P>(v + ((long long)(k + u) * B2 + e) * kSlice) : V(0);
     T xs[U][B];
 #pragma unroll
     for (int u = 0; u < U; u++)
@@ -185,7 +205,7 @@ __device__ __forceinline__ void load_cols2(bool wide, bool uniform, const int2* 
 // longer length.
 // The entries of the multiplied vector come from xf(i) (i = column*B + l):
 // a plain gather, or a value computed from other vectors (see sell_row2).
-template <int B, int U, bool kCols16 = true, class XF>
+template <int B, int U, bool kCols16 = true, int P = kStreamOnce, class XF>
 __device__ __forceinline__ void sell_row2_f(const SellView2& A, const XF xf, int t, float (&y0)[B], float (&y1)[B]) {
   constexpr int B2 = B * B;
   const int r0 = 2 * t;
@@ -211,7 +231,7 @@ __device__ __forceinline__ void sell_row2_f(const SellView2& A, const XF xf, int
 #pragma unroll
     for (int u = 0; u < U; u++)
 #pragma unroll
-      for (int e = 0; e < B2; e++) a[u][e] = ld_stream2(v + ((long long)(k + u) * B2 + e) * 32);
+      for (int e = 0; e < B2; e++) a[u][e] = ld_mat<P>(v + ((long long)(k + u) * B2 + e) * 32);
 #pragma unroll
     for (int u = 0; u < U; u++) {
       float x0[B], x1[B];
@@ -239,7 +259,7 @@ __device__ __forceinline__ void sell_row2_f(const SellView2& A, const XF xf, int
     for (int u = 0; u < U; u++)
 #pragma unroll
       for (int e = 0; e < B2; e++)
-        a[u][e] = u < rem ? ld_stream2(v + ((long long)(k + u) * B2 + e) * 32) : make_float2(0.f, 0.f);
+        a[u][e] = u < rem ? ld_mat<P>(v + ((long long)(k + u) * B2 + e) * 32) : make_float2(0.f, 0.f);
     float x0[U][B], x1[U][B];
 #pragma unroll
     for (int u = 0; u < U; u++)

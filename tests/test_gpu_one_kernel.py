@@ -1,0 +1,152 @@
+"""FP64 CG and BiCGSTAB and refined CG as one cooperative kernel (small and middle systems) against
+the same solves with a kernel per phase, which timing mode runs
+(MONOLIS_B200_PRM_I_KERNEL_TIMERS).
+
+FP64: both sum their dot products in double-double, so iterations and solution
+are the same bits. FP32-refined CG: the plain FP64 sums of the loop differ by
+their grouping, so the counts may differ a little (a refresh moved by an
+iteration: 2) and each side must reach the tolerance on its FP64 residual
+(1.01e-8: the norm is computed here in another order)."""
+import numpy as np
+import pytest
+
+from monolis_b200 import api
+from monolis_b200 import problems as P
+from helpers import bits_equal
+
+pytestmark = pytest.mark.gpu
+
+
+def grid_system(dims, ndof, seed, shuffle=False, skew=0.0):
+    """7-point stencil on a grid of dims points with ndof x ndof blocks,
+    diagonally dominant; skew != 0: nonsymmetric; shuffle: random numbering."""
+    nx, ny, nz = dims
+    n = nx * ny * nz
+    rng = np.random.default_rng(seed)
+    ids = np.arange(n).reshape(nz, ny, nx)
+    pairs = [(ids[:, :, :-1], ids[:, :, 1:]), (ids[:, :-1], ids[:, 1:]), (ids[:-1], ids[1:])]
+    i = np.concatenate([np.arange(n)] + [a.ravel() for a, _ in pairs] + [b.ravel() for _, b in pairs])
+    j = np.concatenate([np.arange(n)] + [b.ravel() for _, b in pairs] + [a.ravel() for a, _ in pairs])
+    m = (len(i) - n) // 2
+    w = -np.exp(0.3 * rng.standard_normal(m))
+    val = np.zeros((len(i), ndof, ndof))
+    for r in range(ndof):
+        val[n:n + m, r, r] = w * (1 + 0.1 * r) * (1 + skew)
+        val[n + m:, r, r] = w * (1 + 0.1 * r) * (1 - skew)
+    coupling = 0.1 * rng.standard_normal((ndof, ndof))
+    val[:n] = coupling + coupling.T
+    diag = 0.05 + np.bincount(i[n:], weights=np.abs(val[n:]).sum(axis=2).max(axis=1), minlength=n) + 0.5 * ndof
+    val[np.arange(n), :, :] += diag[:, None, None] * np.eye(ndof)
+    if shuffle:
+        perm = rng.permutation(n)
+        i, j = perm[i], perm[j]
+    order = np.lexsort((j, i))
+    index = np.concatenate([[0], np.cumsum(np.bincount(i, minlength=n))]).astype(np.int32)
+    return index, j[order].astype(np.int32), np.ascontiguousarray(val[order]), rng.uniform(0.0, 1.0, n * ndof)
+
+
+def device_solve(m, b, timers, offset=0):
+    import torch
+    m.Iarray[api.B200_PRM_I_KERNEL_TIMERS] = int(timers)
+    d_b = torch.from_numpy(b).cuda()
+    d_x = torch.full((len(b) + 2,), 7.0, dtype=torch.float64, device="cuda")  # init_x: overwritten
+    torch.cuda.synchronize()
+    rc = m.device_solve(d_b.data_ptr(), d_x.data_ptr() + 8 * offset)
+    torch.cuda.synchronize()
+    return rc, d_x.cpu().numpy()[offset:offset + len(b)], m.get_converge_iter()
+
+
+# edges of slices (32 rows, 64 in FP32), of 16-byte row groups and of the split
+# over the blocks; a grid whose window does not fit (random numbering); blocks
+# of every size, with more and fewer slices than warps
+@pytest.mark.parametrize("dims,ndof,shuffle", [
+    ((1, 1, 1), 1, False), ((31, 1, 1), 1, False), ((33, 1, 1), 3, False), ((13, 5, 1), 1, False), ((5, 5, 5), 2, False),
+    ((16, 16, 37), 1, False), ((17, 29, 11), 3, False), ((23, 19, 11), 2, False), ((40, 37, 31), 1, False),
+    ((40, 37, 31), 1, True), ((25, 21, 19), 3, True), ((11, 12, 13), 4, False), ((9, 11, 12), 5, False),
+    ((12, 11, 9), 6, False),
+])
+@pytest.mark.parametrize("method,precision", [(api.ITER_CG, 0), (api.ITER_CG, 1), (api.ITER_BICGSTAB, 0)])
+def test_one_kernel_matches_kernels_per_phase(gpu, dims, ndof, shuffle, method, precision):
+    index, item, val, b = grid_system(dims, ndof, 11, shuffle, skew=0.3 if method == api.ITER_BICGSTAB else 0.0)
+    n = len(index) - 1
+    m = api.Monolis(gpu)
+    m.set_matrix_BCSR(n, n, ndof, len(item), val.reshape(-1), index, item)
+    m.quiet()
+    m.set_error_abort(False)
+    m.set_method(method)
+    m.set_precision(precision)
+    m.set_tolerance(1e-8)
+    m.set_maxiter(2000)
+    m.Iarray[api.B200_PRM_I_ITER_RR] = 7  # replacement iterations on the way
+    m.device_prepare()
+    rc0, x0, it0 = device_solve(m, b, True)
+    for offset in (0, 1):  # x on a 16-byte boundary, and not
+        rc1, x1, it1 = device_solve(m, b, False, offset)
+        assert rc1 == rc0
+        if rc0:  # one row: BiCGSTAB divides by the exact zero residual on either path
+            assert n == 1
+            continue
+        if precision == 0:
+            assert it1 == it0 and bits_equal(x1, x0)
+        else:
+            assert abs(it1 - it0) <= 2, (it0, it1)
+            rows = np.repeat(np.arange(n), np.diff(index))
+            ax = np.zeros((n, ndof))
+            np.add.at(ax, rows, np.einsum("krc,kc->kr", val, x1.reshape(n, ndof)[item]))
+            assert np.linalg.norm(b - ax.reshape(-1)) / np.linalg.norm(b) < 1.01e-8
+
+
+def test_one_kernel_initial_guess_log_and_limits(gpu):
+    """Start from a given x, the residual log, max_iter and a zero right-hand
+    side behave as with a kernel per phase."""
+    import torch
+    index, item, val, b = grid_system((14, 13, 12), 1, 3)
+    n = len(index) - 1
+    m = api.Monolis(gpu)
+    m.set_matrix_BCSR(n, n, 1, len(item), val.reshape(-1), index, item)
+    m.quiet()
+    m.set_error_abort(False)
+    m.set_tolerance(1e-10)
+    m.device_prepare()
+    m.set_init_x(False)
+    d_b = torch.from_numpy(b).cuda()
+    out = []
+    for timers in (1, 0):
+        m.Iarray[api.B200_PRM_I_KERNEL_TIMERS] = timers
+        d_x = torch.from_numpy(np.linspace(-1.0, 1.0, n)).cuda()
+        m.show_iterlog(True)
+        assert m.device_solve(d_b.data_ptr(), d_x.data_ptr()) == 0
+        m.show_iterlog(False)
+        out.append((d_x.cpu().numpy(), m.get_converge_iter(), m.get_converge_residual()))
+    assert bits_equal(out[0][0], out[1][0]) and out[0][1:] == out[1][1:]
+    m.set_maxiter(3)
+    assert m.device_solve(d_b.data_ptr(), d_x.data_ptr()) == 1 and m.get_converge_iter() == 3
+    zero = torch.zeros_like(d_b)
+    m.set_init_x(True)
+    assert m.device_solve(zero.data_ptr(), d_x.data_ptr()) == 0
+    assert not d_x.cpu().numpy().any()
+
+
+@pytest.mark.parametrize("method", [api.ITER_CG, api.ITER_BICGSTAB])
+def test_one_kernel_wait_runs_out(gpu, method):
+    """Every wait of the grid is bounded: with 2,000 polls and block 0 starting
+    20 ms late (a bounded sleep) the solve returns MONOLIS_B200_TIMEOUT (4), and
+    the next solve on the same device succeeds."""
+    n = 14
+    m = api.Monolis(gpu)
+    b = P.convection_diffusion(m, n=n, peclet=0.5)
+    m.quiet()
+    m.set_error_abort(False)
+    m.set_method(method)
+    m.set_maxiter(500)
+    m.set_tolerance(1e-6)
+    m.device_prepare()
+    m.Iarray[api.B200_PRM_I_WAIT_LIMIT] = 2000
+    m.Iarray[api.B200_PRM_I_WAIT_DELAY_US] = 20000
+    rc, _, _ = device_solve(m, b, False)
+    assert rc == 4
+    m.Iarray[api.B200_PRM_I_WAIT_LIMIT] = 0
+    m.Iarray[api.B200_PRM_I_WAIT_DELAY_US] = 0
+    rc, x, it = device_solve(m, b, False)
+    rc0, x0, it0 = device_solve(m, b, True)
+    assert rc == rc0 and it == it0 and bits_equal(x, x0)
