@@ -138,6 +138,17 @@ __global__ void element_gradient_generic_kernel(int n_elem, int n_base, int ndof
   }
 }
 
+int transpose_values(SellMatrix& at, const SellMatrix& a, cudaStream_t s) {
+  int rc = dispatch_ndof(a.ndof, [&](auto Bc) {
+    constexpr int B = decltype(Bc)::value;
+    transpose_values_kernel<B><<<148 * 16, 256, 0, s>>>(at.d_perm, a.nz, a.d_csrval, at.d_csrval);
+    return kOk;
+  });
+  if (rc) return rc;
+  MB_CUDA_OK(cudaGetLastError());
+  return kOk;
+}
+
 }  // namespace
 
 int sell_build_transpose(SellMatrix& at, const SellMatrix& a, const int* h_csc_index, const int* h_csc_item,
@@ -151,20 +162,17 @@ int sell_build_transpose(SellMatrix& at, const SellMatrix& a, const int* h_csc_i
   MB_CUDA_OK(grow_buf(&at.d_rowptr, at.cap_rowptr, (size_t)a.N + 1));
   MB_CUDA_OK(grow_buf(&at.d_item, at.cap_item, (size_t)nz));
   MB_CUDA_OK(grow_buf(&at.d_csrval, at.cap_csrval, (size_t)nz * B2));
-  int* d_perm = nullptr;
-  MB_CUDA_OK(cudaMallocAsync((void**)&d_perm, sizeof(int) * (nz + 1), s));
+  MB_CUDA_OK(grow_buf(&at.d_perm, at.cap_perm, (size_t)nz));
   MB_CUDA_OK(cudaMemcpyAsync(at.d_rowptr, h_csc_index, sizeof(int) * (a.N + 1), cudaMemcpyHostToDevice, s));
   MB_CUDA_OK(cudaMemcpyAsync(at.d_item, h_csc_item, sizeof(int) * nz, cudaMemcpyHostToDevice, s));
-  MB_CUDA_OK(cudaMemcpyAsync(d_perm, h_csc_perm, sizeof(int) * nz, cudaMemcpyHostToDevice, s));
-  int rc = dispatch_ndof(a.ndof, [&](auto Bc) {
-    constexpr int B = decltype(Bc)::value;
-    transpose_values_kernel<B><<<148 * 16, 256, 0, s>>>(d_perm, nz, a.d_csrval, at.d_csrval);
-    return kOk;
-  });
-  cudaFreeAsync(d_perm, s);
-  if (rc) return rc;
-  MB_CUDA_OK(cudaGetLastError());
-  return sell_layout(at, s);
+  MB_CUDA_OK(cudaMemcpyAsync(at.d_perm, h_csc_perm, sizeof(int) * nz, cudaMemcpyHostToDevice, s));
+  int rc = transpose_values(at, a, s);
+  return rc ? rc : sell_layout(at, s);
+}
+
+int sell_refill_transpose(SellMatrix& at, const SellMatrix& a, cudaStream_t s) {
+  int rc = transpose_values(at, a, s);
+  return rc ? rc : sell_refill(at, s);
 }
 
 int outer_product64(const SellMatrix& m, const double* lam, const double* x, double scale, double* G,

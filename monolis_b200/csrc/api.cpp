@@ -252,7 +252,8 @@ std::unordered_map<const MONOLIS_COM*, void*>& nccl_comms() {
 struct DevState {
   mb::SellMatrix A;
   mb::SellMatrix AT;  // A^T, built on demand from A's device CSR and the CSC arrays
-  long long build_id = 0, at_build_id = -1;
+  long long build_id = 0, at_build_id = -1;      // contents of A; those A^T was made from
+  long long pattern_id = 0, at_pattern_id = -1;  // the same for the nonzero pattern
   mb::MultiState* multi = nullptr;  // many-right-hand-side solver buffers
   mb::ShardPlan shard;              // multi-rank solve: halo buffers and tables
   bool device_values = false;       // the device values were assembled on the device (not uploaded)
@@ -388,6 +389,7 @@ int prepare(MONOLIS* m, DevState* s, bool need_diag, bool need_fp32, double* t_h
     s->key_version = I[MONOLIS_B200_PRM_I_MATRIX_VERSION];
     s->prepared = true;
     s->build_id++;
+    s->pattern_id++;
   }
   if (need_diag && !s->A.have_alu) {
     int rc = mb::diag_setup(s->A, st);
@@ -417,7 +419,15 @@ int prepare_transpose(MONOLIS* m, DevState* s, bool need_diag, bool need_fp32) {
     return mb::kBadInput;
   }
   cudaStream_t st = ctx().stream;
+  if (s->at_build_id != s->build_id && s->at_pattern_id == s->pattern_id) {
+    // values assembled on the device: A^T's pattern and layout stay
+    s->at_build_id = -1;
+    int rc = mb::sell_refill_transpose(s->AT, s->A, st);
+    if (rc) return rc;
+    s->at_build_id = s->build_id;
+  }
   if (s->at_build_id != s->build_id) {
+    s->at_pattern_id = -1;
     const int* ci = a->CSC.index;
     const int* cit = a->CSC.item;
     const int* cp = a->CSC.perm;
@@ -435,6 +445,7 @@ int prepare_transpose(MONOLIS* m, DevState* s, bool need_diag, bool need_fp32) {
     int rc = mb::sell_build_transpose(s->AT, s->A, ci, cit, cp, st);
     if (rc) return rc;
     s->at_build_id = s->build_id;
+    s->at_pattern_id = s->pattern_id;
   }
   if (need_diag && !s->AT.have_alu) {
     int rc = mb::diag_setup(s->AT, st);
@@ -1205,11 +1216,9 @@ int monolis_b200_solve_multi_R(MONOLIS* m, MONOLIS_COM* com, int n_rhs, double* 
 
 // ---- device assembly ----
 namespace {
-// Device values changed: rebuild the SELL values (FP32 copy, DIAG factors and
+// Device values changed, the layout's with them (FP32 copy, DIAG factors and
 // the transpose follow on demand).
 int after_device_assembly(MONOLIS* m, DevState* s) {
-  int rc = mb::sell_layout(s->A, ctx().stream);
-  if (rc) return rc;
   s->device_values = true;
   s->build_id++;
   s->key_version = m->prm.Iarray[MONOLIS_B200_PRM_I_MATRIX_VERSION];
@@ -1223,8 +1232,8 @@ int monolis_b200_device_clear_matrix(MONOLIS* m) {
   DevState* s = state_of(m);
   int rc = prepare(m, s, false, false, nullptr);
   if (rc) return rc;
-  const size_t nv = (size_t)s->A.nz * m->mat.NDOF * m->mat.NDOF;
-  MB_API_CUDA(cudaMemsetAsync(s->A.d_csrval, 0, nv * sizeof(double), ctx().stream));
+  rc = mb::device_clear_values(s->A, ctx().stream);
+  if (rc) return rc;
   return after_device_assembly(m, s);
 }
 
