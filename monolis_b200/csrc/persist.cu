@@ -1012,7 +1012,7 @@ struct Shape {
   static constexpr int u = B == 1 ? 4 : (B <= 3 ? 3 : 1);
   static constexpr int d = B == 1 ? 3 : 2;
 };
-constexpr int kSmemBytes = 220 * 1024;
+constexpr int kSmemBytes = 220 * 1024, kSmemCache = 180 * 1024;
 // CG keeps P in windows up to this block size; BiCGSTAB and larger blocks
 // gather from global memory. us an iteration, window / no window: CG ndof 3,
 // 33^3 nodes FP64 19.4 / 24.7, 8^3 11.8 / 16.0; ndof 6, 36^3 45.9 / 41.1;
@@ -1050,8 +1050,11 @@ PersistPlan make_plan(const SellMatrix& m, const SolveParams& p) {
   q.window = p.method == 1 && B <= kWindowMaxNdof && meta + win + 64 <= kSmemBytes;
   q.win_rows = q.window ? (int)(win / (B * tsize)) : 0;
   const long long cache = (slots / q.grid + m.wmax + 8) * (32LL * (B * B * 8 + (mixed ? 8 : 4)));  // about a block's part of the matrix
-  const long long want = meta + (q.window ? up16((int)win) : 0) + (long long)nown * own_bytes + cache;
-  q.smem = (int)std::min<long long>(want, kSmemBytes);
+  // slices of the matrix up to kSmemCache only: beyond it they cost the loads
+  // in flight more L1 than they save (57x49x61 nodes refined, 180 KB 43.4 us
+  // an iteration, 220 KB 46.1; 33^3 FP64 18.3 and 19.2)
+  const long long need = meta + (q.window ? up16((int)win) : 0) + (long long)nown * own_bytes;
+  q.smem = (int)std::min<long long>(kSmemBytes, std::max(need, std::min<long long>(need + cache, kSmemCache)));
   q.ok = meta <= kSmemBytes;
   return q;
 }
