@@ -144,7 +144,9 @@ __device__ __forceinline__ int find_slot(const int* __restrict__ rowptr, const i
 // by one lane. What bounds it is the element matrices and the values, each
 // read or written once: 70,110 nodes of 3 dofs, a matrix per element (300 MB
 // in, 130 MB in and out), took 1850 us with a thread per row that searched
-// the row's columns for every (a, b).
+// the row's columns for every (a, b), 650 us with a warp per row taking one
+// element at a time (each waits for its loads), about 300 us with the loads of
+// kGroup elements in flight (whole call 3240 -> 782 -> 425 us).
 template <int B>
 __global__ void __launch_bounds__(256) add_elements_kernel(const int* __restrict__ rowptr, const int* __restrict__ item,
                                                            int N, const int* __restrict__ iptr, int* __restrict__ ilist,
@@ -152,7 +154,7 @@ __global__ void __launch_bounds__(256) add_elements_kernel(const int* __restrict
                                                            const double* __restrict__ val, long long val_stride,
                                                            const double* __restrict__ scale, double* __restrict__ A,
                                                            int* __restrict__ bad) {
-  constexpr int B2 = B * B;
+  constexpr int B2 = B * B, kGroup = B <= 2 ? 4 : (B <= 4 ? 2 : 1);
   constexpr unsigned kAll = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const int i = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
@@ -198,34 +200,71 @@ __global__ void __launch_bounds__(256) add_elements_kernel(const int* __restrict
 #pragma unroll
       for (int e = 0; e < B2; e++) acc[e] = dst[e];
     }
-    for (int q = 0; q < nq; q++) {
-      const long long e = nq <= 32 ? __shfl_sync(kAll, mine, q) : ilist[q0 + q];
-      const int* en = elem + e * n_base;
-      const double* Ke = val + e * val_stride;
-      const double s = scale ? scale[e] : 1.0;
-      for (int a0 = 0; a0 < n_base; a0 += 32) {
-        const int va = a0 + lane < n_base ? en[a0 + lane] : -1;
-        unsigned rows = __ballot_sync(kAll, va == i);
-        while (rows) {
-          const int a = a0 + __ffs(rows) - 1;
-          rows &= rows - 1;
+    // kGroup elements at a time: their connectivities, then the values each
+    // lane takes from them, are in flight together; added in element order
+    for (int q = 0; q < nq; q += kGroup) {
+      long long e[kGroup];
+      int va[kGroup];
+      unsigned hit[kGroup], rows[kGroup];  // b with this lane's column, a with this row
+      bool plain = n_base <= 32;
+#pragma unroll
+      for (int g = 0; g < kGroup; g++) {
+        const int qg = min(q + g, nq - 1);
+        e[g] = nq <= 32 ? __shfl_sync(kAll, mine, qg) : ilist[q0 + qg];
+        va[g] = q + g < nq && lane < n_base ? elem[e[g] * n_base + lane] : -1;
+      }
+#pragma unroll
+      for (int g = 0; g < kGroup; g++) {
+        rows[g] = __ballot_sync(kAll, va[g] == i);
+        hit[g] = 0;
+        for (int t = 0; t < min(n_base, 32); t++)
+          if (__shfl_sync(kAll, va[g], t) == col) hit[g] |= 1u << t;
+        if (q + g >= nq || col < 0) hit[g] = 0;
+        // a node once in the element (and one 32-lane load of its nodes)
+        plain = plain && __popc(rows[g]) <= 1 && !__any_sync(kAll, __popc(hit[g]) > 1);
+      }
+      if (plain) {
+        double v[kGroup][B2], sc[kGroup];
+#pragma unroll
+        for (int g = 0; g < kGroup; g++) {
+          if (rows[g] && kb == k0) want += n_base;
+          if (!rows[g]) hit[g] = 0;
+          if (!hit[g]) continue;
+          got++;
+          const double* Ka =
+              val + e[g] * val_stride + (long long)(__ffs(rows[g]) - 1) * B * ncol + (__ffs(hit[g]) - 1) * B;
+          sc[g] = scale ? scale[e[g]] : 1.0;
+#pragma unroll
+          for (int r = 0; r < B; r++)
+#pragma unroll
+            for (int c = 0; c < B; c++) v[g][r * B + c] = Ka[(long long)r * ncol + c];
+        }
+#pragma unroll
+        for (int g = 0; g < kGroup; g++)
+          if (hit[g]) {
+#pragma unroll
+            for (int x = 0; x < B2; x++) acc[x] = __dadd_rn(acc[x], scale ? __dmul_rn(sc[g], v[g][x]) : v[g][x]);
+          }
+        continue;
+      }
+      for (int g = 0; g < kGroup && q + g < nq; g++) {
+        const long long eg = nq <= 32 ? __shfl_sync(kAll, mine, q + g) : ilist[q0 + q + g];
+        const int* en = elem + eg * n_base;
+        const double s = scale ? scale[eg] : 1.0;
+        for (int a = 0; a < n_base; a++) {
+          if (en[a] != i) continue;
           if (kb == k0) want += n_base;
-          const double* Ka = Ke + (long long)a * B * ncol;
-          for (int b0 = 0; b0 < n_base; b0 += 32) {
-            const int vb = b0 == a0 ? va : (b0 + lane < n_base ? en[b0 + lane] : -1);
-            const int nb = min(32, n_base - b0);
-            for (int t = 0; t < nb; t++) {
-              if (__shfl_sync(kAll, vb, t) != col) continue;
-              got++;
-              const int b = b0 + t;
+          const double* Ka = val + eg * val_stride + (long long)a * B * ncol;
+          for (int t = 0; t < n_base; t++) {
+            if (en[t] != col) continue;
+            got++;
 #pragma unroll
-              for (int r = 0; r < B; r++)
+            for (int r = 0; r < B; r++)
 #pragma unroll
-                for (int c = 0; c < B; c++) {
-                  const double v = Ka[(long long)r * ncol + b * B + c];
-                  acc[r * B + c] = __dadd_rn(acc[r * B + c], scale ? __dmul_rn(s, v) : v);
-                }
-            }
+              for (int c = 0; c < B; c++) {
+                const double v = Ka[(long long)r * ncol + t * B + c];
+                acc[r * B + c] = __dadd_rn(acc[r * B + c], scale ? __dmul_rn(s, v) : v);
+              }
           }
         }
       }

@@ -1,0 +1,128 @@
+"""Device assembly at the sizes where the warp-per-row kernels change their way:
+rows of more than 32 blocks, nodes of more than 32 elements, elements of more
+than 32 nodes, a node twice in an element, a column stored twice in a row,
+conditions repeated on a dof. Bit-identical to the host calls made in order."""
+import numpy as np
+import pytest
+
+from monolis_b200 import api
+from helpers import bits_equal
+
+pytestmark = pytest.mark.gpu
+
+
+def meshes():
+    rng = np.random.default_rng(3)
+    star = np.stack([np.zeros(50, dtype=int), np.arange(1, 51)], axis=1)  # node 0: 51 blocks, 50 elements
+    tris = rng.integers(0, 40, (90, 3))  # repeated nodes in some elements, many elements a node
+    tris[:5, 2] = tris[:5, 0]
+    big = np.stack([rng.permutation(80)[:40] for _ in range(6)])  # 40 nodes an element
+    big[0, 39] = big[0, 0]
+    chain = np.stack([np.arange(0, 200), np.arange(1, 201)], axis=1)
+    return {"star": (51, star), "tris": (40, tris), "big": (80, big), "chain": (201, chain)}
+
+
+def device_values(m, lib):
+    v = np.empty(m.NZ * m.NDOF ** 2)
+    assert lib.monolis_b200_device_get_values(m.p, v.ctypes.data_as(api._dp)) == 0
+    return v
+
+
+def setup(gpu, name, ndof):
+    n, elem = meshes()[name]
+    ms = []
+    for _ in range(2):
+        m = api.Monolis(gpu)
+        m.get_nonzero_pattern_flat(n, elem.shape[1], ndof, elem)
+        m.quiet()
+        ms.append(m)
+    return n, np.ascontiguousarray(elem, dtype=np.int32), ms
+
+
+@pytest.mark.parametrize("name", ["star", "tris", "big", "chain"])
+@pytest.mark.parametrize("ndof,scaled,own", [(1, True, False), (2, False, True), (3, True, True), (6, False, False)])
+def test_rows_and_conditions_match_host(gpu, name, ndof, scaled, own):
+    import torch
+    n, elem, (mh, md) = setup(gpu, name, ndof)
+    rng = np.random.default_rng(7)
+    ne, nb = elem.shape
+    size = (nb * ndof) ** 2
+    val = rng.standard_normal(size * (ne if own else 1))
+    scale = rng.standard_normal(ne) if scaled else None
+    mh.add_elements(elem, nb, val, size if own else 0, scale=scale)
+    mh.add_elements(elem, nb, val, size if own else 0, scale=scale)
+    d_elem, d_val = torch.from_numpy(elem).cuda(), torch.from_numpy(val).cuda()
+    d_scale = torch.from_numpy(scale).cuda() if scaled else None
+    torch.cuda.synchronize()
+    assert gpu.monolis_b200_device_clear_matrix(md.p) == 0
+    for _ in range(2):
+        assert gpu.monolis_b200_device_add_elements_R(md.p, ne, nb, d_elem.data_ptr(), d_val.data_ptr(),
+                                                      size if own else 0, d_scale.data_ptr() if scaled else None) == 0
+    assert bits_equal(device_values(md, gpu), mh.values())
+    # conditions on every fifth node, the first one three times
+    nodes = np.array(list(range(0, n, 5)) + [0, 0], dtype=np.int32)
+    dofs = (np.arange(len(nodes)) % ndof).astype(np.int32)
+    dofs[-2:] = 0
+    vals = rng.standard_normal(len(nodes))
+    b = rng.standard_normal(n * ndof)
+    d_b = torch.from_numpy(b).cuda()
+    torch.cuda.synchronize()
+    for q in range(len(nodes)):
+        mh.set_Dirichlet_bc(b, nodes[q], dofs[q], vals[q])
+    assert gpu.monolis_b200_device_set_Dirichlet_bc_R(md.p, d_b.data_ptr(), len(nodes), nodes.ctypes.data_as(api._ip),
+                                                      dofs.ctypes.data_as(api._ip), vals.ctypes.data_as(api._dp)) == 0
+    assert bits_equal(device_values(md, gpu), mh.values())
+    assert bits_equal(d_b.cpu().numpy(), b)
+    # the layout the products read has the same values, A^T too (before and
+    # after a second assembly on an unchanged pattern)
+    x = rng.standard_normal(n * ndof)
+    for again in (False, True):
+        if again:
+            mh.add_elements(elem, nb, val, size if own else 0, scale=scale)
+            assert gpu.monolis_b200_device_add_elements_R(md.p, ne, nb, d_elem.data_ptr(), d_val.data_ptr(),
+                                                          size if own else 0,
+                                                          d_scale.data_ptr() if scaled else None) == 0
+        d_x, d_y = torch.from_numpy(x).cuda(), torch.zeros(n * ndof, dtype=torch.float64, device="cuda")
+        torch.cuda.synchronize()
+        md.device_matvec(d_x.data_ptr(), d_y.data_ptr())
+        torch.cuda.synchronize()
+        assert bits_equal(d_y.cpu().numpy(), mh.matvec(x))
+        assert gpu.monolis_b200_device_matvec_transpose_R(md.p, d_x.data_ptr(), d_y.data_ptr()) == 0
+        torch.cuda.synchronize()
+        assert bits_equal(d_y.cpu().numpy(), mh.matvec_transpose(x))
+
+
+def test_column_stored_twice(gpu):
+    """A nodal graph that lists the node itself stores its column twice; both
+    sides add to the block their binary search finds."""
+    import torch
+    n = 37
+    index = np.arange(0, 3 * n + 1, 3, dtype=np.int32)
+    item = np.stack([(np.arange(n) - 1) % n, np.arange(n), (np.arange(n) + 1) % n], axis=1).astype(np.int32).reshape(-1)
+    elem = np.stack([np.arange(n), (np.arange(n) + 1) % n], axis=1).astype(np.int32)
+    val = np.random.default_rng(5).standard_normal(4)
+    ms = []
+    for _ in range(2):
+        m = api.Monolis(gpu)
+        m.get_nonzero_pattern_by_nodal_graph(n, 1, index, item)
+        m.quiet()
+        ms.append(m)
+    ms[0].add_elements(elem, 2, val, 0)
+    d_elem, d_val = torch.from_numpy(elem).cuda(), torch.from_numpy(val).cuda()
+    torch.cuda.synchronize()
+    assert gpu.monolis_b200_device_clear_matrix(ms[1].p) == 0
+    assert gpu.monolis_b200_device_add_elements_R(ms[1].p, n, 2, d_elem.data_ptr(), d_val.data_ptr(), 0, None) == 0
+    assert bits_equal(device_values(ms[1], gpu), ms[0].values())
+
+
+def test_bad_elements_leave_the_values(gpu):
+    """A node out of range is refused and nothing is added."""
+    import torch
+    n, elem, (_, m) = setup(gpu, "chain", 1)
+    bad = elem.copy()
+    bad[17, 1] = n
+    d_elem, d_val = torch.from_numpy(bad).cuda(), torch.ones(4, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    assert gpu.monolis_b200_device_clear_matrix(m.p) == 0
+    assert gpu.monolis_b200_device_add_elements_R(m.p, len(bad), 2, d_elem.data_ptr(), d_val.data_ptr(), 0, None) == 5
+    assert not device_values(m, gpu).any()
