@@ -5,13 +5,15 @@
 // + k] for right-hand side k < K <= 32, so that a warp owns one block row and
 // lane k works on right-hand side k: every vector access of the warp is one
 // contiguous line, and the matrix row (CSR, read once for all K) is loaded
-// cooperatively by the lanes and broadcast with shuffles. One warp keeps the
-// same rows in every phase, so a thread only ever reads back the entries it
-// wrote itself; values of other rows (the SpMV gathers) are read through L2.
+// cooperatively by the lanes and broadcast with shuffles. A block owns a
+// contiguous run of rows and a warp the same rows of it in every phase, so a
+// thread only ever reads back the entries it wrote itself; the gathers of the
+// product go through L1 (each barrier makes the SM refetch), where the
+// neighbours that lie in the block's own run are found again.
 //
 // The kernel is launched cooperatively (all blocks resident) and separates
 // its phases with a grid barrier whose last arriving block also sums the
-// per-block partial dot products (block order: deterministic) and updates the
+// per-block partial dot products (fixed order: deterministic) and updates the
 // per-right-hand-side scalars before releasing the others. Each barrier wait
 // is bounded: past the limit a block records an error and every block leaves.
 // Two barriers per iteration: the search direction p = z + beta p is formed
@@ -34,22 +36,28 @@ namespace mb {
 namespace {
 
 constexpr int kMultiK = 32;
-constexpr int kMultiThreads = 256;
-// default bound of every barrier wait: polls of an L2 round trip + 32 ns each, seconds in all
+// default bound of every barrier wait: polls of an L2 round trip, seconds in all
 constexpr unsigned long long kSpinLimit = 1ull << 22;
 
-constexpr int kBarrierGroup = 32;  // blocks per first-level group of the barrier
-constexpr int kMaxGroups = 128;
-
-constexpr int kLine = 32;  // words per 128-byte line: every counter and flag gets its own
+// Threads of a block. Matrices of 1x1 and 2x2 blocks run one block to an SM, so
+// that an SM's rows are one run and the barrier has few arrivals: 768 threads
+// of 80 registers, or in FP32, where an iteration's vectors do not stay in L2
+// (kStride), 1024 of 64 (more loads in flight for HBM; they spill a little).
+// Larger blocks run as many blocks as fit. us an iteration, 768 / 1024
+// threads, 7-entry rows, FP32: 50^3 x 32 right-hand sides 78.8 / 81.7, 30^3 x 5
+// 30.0 / 34.7, 96^3 x 32 430 / 383; the form before (592 blocks of 256 threads,
+// a two-level barrier, gathers past L1, no prefetch) 83, 37 and 382, 12^3 x 32
+// 44 against 29; FP64 96^3 x 32 716 against 650.
+template <int B, class T, bool kStride>
+struct MultiShape {
+  static constexpr int threads = B > 2 ? 256 : (sizeof(T) == 4 && kStride ? 1024 : 768);
+};
 
 struct MultiCtl {
-  alignas(128) unsigned int count;  // groups finished (global arrival)
-  alignas(128) unsigned int gen;    // global release generation
+  alignas(128) unsigned int count;  // blocks arrived
+  alignas(128) unsigned int gen;    // release generation
   alignas(128) int err;
   int all_done, any_refresh, it;
-  alignas(128) unsigned int gcount[kMaxGroups * kLine];  // blocks arrived, per group
-  alignas(128) unsigned int grel[kMaxGroups * kLine];    // release generation, per group
   double rho[kMultiK], rho1[kMultiK], alpha[kMultiK], beta[kMultiK], B2[kMultiK], rmax[kMultiK], resid[kMultiK];
   int iter[kMultiK], done[kMultiK], status[kMultiK], refresh[kMultiK], fold[kMultiK], nref[kMultiK];
 };
@@ -81,90 +89,61 @@ __device__ __forceinline__ void st_release(unsigned int* p, unsigned int v) {
   asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
+__device__ __forceinline__ void fence_gpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
+
 // Grid barrier of a cooperative launch, with an optional reduction of the
-// per-block partial sums (2 x 32 doubles per block, partials[block][64]).
-// Blocks arrive in groups of kBarrierGroup: the last block of a group sums
-// the group's partials in block order (group sums after the block partials),
-// the last group finisher sums the group sums in group order into tot and
-// runs `last` (with all its threads) before releasing everyone. Each block
-// adds at most one group's worth of values, so the barrier's tail stays short.
-// Waits are bounded; returns false once any block has given up.
-template <class F>
-__device__ bool grid_sync(MultiCtl* c, double* partials, bool reduce, double (*tot)[kMultiK],
+// per-block partial sums (2 x 32 doubles per block, partials[block][64]): the
+// last block to arrive adds them, TH/64 strided parts of every sum and then the
+// parts in order, into tot and runs `last` (with all its threads) before
+// releasing everyone. One counter and one release word: 148 arrivals and
+// pollers are cheaper than a level of groups between. Waits are bounded;
+// returns false once any block has given up.
+template <int TH, class F>
+__device__ bool grid_sync(MultiCtl* c, double* partials, bool reduce, double (*tot)[kMultiK], double* parts /* TH */,
                           unsigned long long limit, F&& last) {
-  __shared__ unsigned int s_grel, s_gen;
-  __shared__ int s_role, s_ok;  // 0: wait for the group, 1: group finisher, 2: last block
-  const unsigned int G = gridDim.x, g = blockIdx.x / kBarrierGroup;
-  const unsigned int ngroups = (G + kBarrierGroup - 1) / kBarrierGroup;
-  const unsigned int g0 = g * kBarrierGroup, gsize = min((unsigned int)kBarrierGroup, G - g0);
-  unsigned int* gcount = c->gcount + g * kLine;
-  unsigned int* grel = c->grel + g * kLine;
-  double* gpart = partials + (size_t)G * 2 * kMultiK;
+  __shared__ unsigned int s_gen;
+  __shared__ int s_last, s_ok;
+  const unsigned int G = gridDim.x;
   __syncthreads();
   if (threadIdx.x == 0) {
-    s_grel = ld_acquire(grel);
     s_gen = ld_acquire(&c->gen);
-    __threadfence();
-    s_role = atomicAdd(gcount, 1u) == gsize - 1 ? 1 : 0;
+    fence_gpu();
+    s_last = atomicAdd(&c->count, 1u) == G - 1;
   }
   __syncthreads();
-  if (s_role == 1) {
-    __threadfence();
-    if (reduce && threadIdx.x < 2 * kMultiK) {
+  if (s_last) {
+    fence_gpu();
+    if (reduce) {
+      constexpr int W = 2 * kMultiK, NP = TH / W;
+      const int w = threadIdx.x % W, q = threadIdx.x / W;
       double s = 0.0;
-#pragma unroll 8
-      for (unsigned int b = 0; b < gsize; b++) s += __ldcg(partials + (size_t)(g0 + b) * 2 * kMultiK + threadIdx.x);
-      gpart[(size_t)g * 2 * kMultiK + threadIdx.x] = s;
+#pragma unroll 4
+      for (unsigned int b = q; b < G; b += NP) s += __ldcg(partials + (size_t)b * W + w);
+      parts[threadIdx.x] = s;
+      __syncthreads();
+      if (threadIdx.x < W) {
+        double t = 0.0;
+#pragma unroll
+        for (int k = 0; k < NP; k++) t += parts[k * W + threadIdx.x];
+        tot[threadIdx.x >> 5][threadIdx.x & 31] = t;
+      }
+      __syncthreads();
     }
+    last();
     __syncthreads();
     if (threadIdx.x == 0) {
-      *gcount = 0u;
-      __threadfence();
-      if (atomicAdd(&c->count, 1u) == ngroups - 1) s_role = 2;
+      c->count = 0u;
+      fence_gpu();
+      st_release(&c->gen, s_gen + 1u);
     }
-    __syncthreads();
-    if (s_role == 2) {
-      __threadfence();
-      if (reduce) {
-        if (threadIdx.x < 2 * kMultiK) {
-          double t = 0.0;
-#pragma unroll 8
-          for (unsigned int q = 0; q < ngroups; q++) t += __ldcg(gpart + (size_t)q * 2 * kMultiK + threadIdx.x);
-          tot[threadIdx.x >> 5][threadIdx.x & 31] = t;
-        }
-        __syncthreads();
-      }
-      last();
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        c->count = 0u;
-        __threadfence();
-        st_release(&c->gen, s_gen + 1u);
-      }
-    } else if (threadIdx.x == 0) {
-      // group finisher: wait for the global release (at most ngroups pollers)
-      unsigned long long n = 0;
-      while (ld_acquire(&c->gen) == s_gen) {
-        if (++n > limit) {
-          atomicExch(&c->err, 1);
-          break;
-        }
-        __nanosleep(32);
-      }
-      __threadfence();
-    }
-    if (threadIdx.x == 0) st_release(grel, s_grel + 1u);  // release this group
   } else if (threadIdx.x == 0) {
-    // wait for this group's release (at most kBarrierGroup pollers per line)
     unsigned long long n = 0;
-    while (ld_acquire(grel) == s_grel) {
+    while (ld_acquire(&c->gen) == s_gen)
       if (++n > limit) {
         atomicExch(&c->err, 1);
         break;
       }
-      __nanosleep(32);
-    }
-    __threadfence();
+    fence_gpu();
   }
   if (threadIdx.x == 0) s_ok = __ldcg(&c->err) == 0;
   __syncthreads();
@@ -179,20 +158,14 @@ template <>
 __device__ __forceinline__ double fmat<double>(double a, double b, double c) { return fma(a, b, c); }
 
 // Four consecutive right-hand sides of one vector entry: one 16-byte access
-// for FP32, two for FP64; kCoherent reads through L2 (values written by other
-// blocks of this launch).
-template <bool kCoherent, class T>
-__device__ __forceinline__ void ld4(const T* p, T (&o)[4]);
-template <bool kCoherent>
+// for FP32, two for FP64.
 __device__ __forceinline__ void ld4(const float* p, float (&o)[4]) {
-  const float4 v = kCoherent ? __ldcg(reinterpret_cast<const float4*>(p)) : *reinterpret_cast<const float4*>(p);
+  const float4 v = *reinterpret_cast<const float4*>(p);
   o[0] = v.x; o[1] = v.y; o[2] = v.z; o[3] = v.w;
 }
-template <bool kCoherent>
 __device__ __forceinline__ void ld4(const double* p, double (&o)[4]) {
   const double2* q = reinterpret_cast<const double2*>(p);
-  const double2 a = kCoherent ? __ldcg(q) : q[0];
-  const double2 b = kCoherent ? __ldcg(q + 1) : q[1];
+  const double2 a = q[0], b = q[1];
   o[0] = a.x; o[1] = a.y; o[2] = b.x; o[3] = b.y;
 }
 __device__ __forceinline__ void st4(float* p, const float (&o)[4]) {
@@ -209,11 +182,11 @@ __device__ __forceinline__ void st4(double* p, const double (&o)[4]) {
 // right-hand sides are zero and start converged). The row's matrix entries are
 // loaded by the group's lanes, Q at a time, and broadcast with width-Q
 // shuffles; all loops that contain shuffles run to warp-uniform bounds.
-// Small blocks are held to few registers (4 blocks of FP32, 3 of FP64 per
-// SM) so that enough loads are in flight for HBM bandwidth.
-template <int B, class T, int Q>
-__global__ void __launch_bounds__(kMultiThreads, B <= 2 ? (sizeof(T) == 4 ? 4 : 3) : 1)
-    multi_cg_kernel(const MultiArgs<T> a) {
+// Small blocks are held to few registers (MultiShape) so that enough loads are
+// in flight.
+template <int B, class T, int Q, bool kStride>
+__global__ void __launch_bounds__(MultiShape<B, T, kStride>::threads, 1) multi_cg_kernel(const MultiArgs<T> a) {
+  constexpr int TH = MultiShape<B, T, kStride>::threads;
   constexpr int B2 = B * B;
   constexpr int Kp = 4 * Q;
   constexpr int RPW = 32 / Q;  // rows per warp
@@ -223,20 +196,24 @@ __global__ void __launch_bounds__(kMultiThreads, B <= 2 ? (sizeof(T) == 4 ? 4 : 
   const double* __restrict__ val64 = a.val64;
   const T* __restrict__ alu = a.alu;
   const double* __restrict__ bv = a.b;
-  double* __restrict__ xv = a.x;
-  T* __restrict__ yv = a.y;
-  T* __restrict__ rv = a.r;
-  T* __restrict__ zv = a.z;
-  T* __restrict__ qv = a.q;
-  __shared__ double s_red[kMultiThreads / 32][2][kMultiK];
+  // written and gathered in this launch: no __restrict__
+  double* xv = a.x;
+  T* yv = a.y;
+  T* rv = a.r;
+  T* zv = a.z;
+  T* qv = a.q;
+  __shared__ double s_red[TH / 32][2][kMultiK];
+  __shared__ double s_parts[TH];
   __shared__ double s_tot[2][kMultiK];
   __shared__ int s_flag[2];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const int qd = lane & (Q - 1);  // quad of right-hand sides
   const int g = lane / Q;         // row slot within the warp
-  const long long wrow0 = ((long long)blockIdx.x * nw + warp) * RPW;  // first row of this warp
-  const long long sweep = (long long)gridDim.x * nw * RPW;
-  const long long N = a.N;
+  // the warp's rows: wrow0, wrow0 + sweep, ... below N, in the block's own run
+  // of rows, or (kStride) among all blocks' rows
+  const long long wrow0 = (kStride ? (long long)blockIdx.x * nw * RPW : (long long)a.N * blockIdx.x / gridDim.x) + warp * RPW;
+  const long long sweep = (kStride ? (long long)gridDim.x : 1LL) * nw * RPW;
+  const long long N = kStride ? a.N : (long long)a.N * (blockIdx.x + 1) / gridDim.x;
   const int K = a.K;
   MultiCtl* c = a.ctl;
   // the last block of a barrier reads and writes the scalars through a
@@ -331,8 +308,8 @@ __global__ void __launch_bounds__(kMultiThreads, B <= 2 ? (sizeof(T) == 4 ? 4 : 
               const long long ij = ((long long)j * B + l) * Kp + 4 * qd;
               double x4[4];
               T y4[4];
-              ld4<true>(xv + ij, x4);
-              ld4<true>(yv + ij, y4);
+              ld4(xv + ij, x4);
+              ld4(yv + ij, y4);
 #pragma unroll
               for (int rr = 0; rr < B; rr++)
 #pragma unroll
@@ -348,10 +325,10 @@ __global__ void __launch_bounds__(kMultiThreads, B <= 2 ? (sizeof(T) == 4 ? 4 : 
         for (int cc = 0; cc < B; cc++) {
           const long long i = at(row, cc);
           double bb[4];
-          ld4<false>(bv + i, bb);
+          ld4(bv + i, bb);
           T r4[4], z4[4];
-          ld4<false>(rv + i, r4);
-          ld4<false>(zv + i, z4);
+          ld4(rv + i, r4);
+          ld4(zv + i, z4);
 #pragma unroll
           for (int j = 0; j < 4; j++) {
             b4[cc][j] = bb[j] - ax[cc][j];
@@ -393,14 +370,14 @@ __global__ void __launch_bounds__(kMultiThreads, B <= 2 ? (sizeof(T) == 4 ? 4 : 
     for (unsigned int t = 0; t < a.delay_ns; t += 1000) __nanosleep(1000);
   }
   // the whole grid has zeroed its x and y before any residual reads them
-  if (!grid_sync(c, a.partials, false, s_tot, a.spin_limit, [] {})) return;
+  if (!grid_sync<TH>(c, a.partials, false, s_tot, s_parts, a.spin_limit, [] {})) return;
   {
     bool all[4];
 #pragma unroll
     for (int j = 0; j < 4; j++) all[j] = 4 * qd + j < K;
     refresh(all);
   }
-  if (!grid_sync(c, a.partials, true, s_tot, a.spin_limit, [&] {
+  if (!grid_sync<TH>(c, a.partials, true, s_tot, s_parts, a.spin_limit, [&] {
         if (threadIdx.x < kMultiK) {
           const int kk = threadIdx.x;
           const double rr = s_tot[0][kk], rz = s_tot[1][kk];
@@ -442,11 +419,29 @@ __global__ void __launch_bounds__(kMultiThreads, B <= 2 ? (sizeof(T) == 4 ? 4 : 
     // P = Z + beta P (own rows, to pnew); Q = A P with the neighbours' P
     // recomputed from Z and the old P; <P,Q>
     double pq[4] = {0.0, 0.0, 0.0, 0.0}, zero4[4] = {0.0, 0.0, 0.0, 0.0};
+    // the next rows' extent and first blocks are loaded ahead, so that a row
+    // waits for its gathers only
+    int k0 = 0, len = 0, cj = 0;
+    T vv[B2];
+    auto extent = [&](long long row, int& k, int& l) {
+      k = row < N ? rowptr[row] : 0;
+      l = row < N ? rowptr[row + 1] - k : 0;
+    };
+    auto blocks = [&](int k, int l, int& col, T(&v)[B2]) {
+      const bool has = qd < l;
+      col = has ? colv[k + qd] : 0;
+#pragma unroll
+      for (int e = 0; e < B2; e++) v[e] = has ? val[(long long)(k + qd) * B2 + e] : T(0);
+    };
+    extent(wrow0 + g, k0, len);
+    blocks(k0, len, cj, vv);
     for (long long rb = wrow0; rb < N; rb += sweep) {
       const long long row = rb + g;
       const bool valid = row < N;
-      const int k0 = valid ? rowptr[row] : 0;
-      const int len = valid ? rowptr[row + 1] - k0 : 0;
+      int k1, len1, cj1;
+      T vv1[B2];
+      extent(row + sweep, k1, len1);
+      blocks(k1, len1, cj1, vv1);
       const int mlen = warp_max(len);
       T acc[B][4];
 #pragma unroll
@@ -454,11 +449,7 @@ __global__ void __launch_bounds__(kMultiThreads, B <= 2 ? (sizeof(T) == 4 ? 4 : 
 #pragma unroll
         for (int j = 0; j < 4; j++) acc[cc][j] = T(0);
       for (int base = 0; base < mlen; base += Q) {
-        const bool has = base + qd < len;
-        const int cj = has ? colv[k0 + base + qd] : 0;
-        T vv[B2];
-#pragma unroll
-        for (int e = 0; e < B2; e++) vv[e] = has ? val[(long long)(k0 + base + qd) * B2 + e] : T(0);
+        if (base) blocks(k0 + base, len - base, cj, vv);
 #pragma unroll
         for (int u = 0; u < Q; u++) {
           const int j = __shfl_sync(0xffffffffu, cj, u, Q);
@@ -470,8 +461,8 @@ __global__ void __launch_bounds__(kMultiThreads, B <= 2 ? (sizeof(T) == 4 ? 4 : 
             for (int l = 0; l < B; l++) {
               const long long ij = ((long long)j * B + l) * Kp + 4 * qd;
               T z4[4], p4[4];
-              ld4<true>(zv + ij, z4);
-              if (!first) ld4<true>(pold + ij, p4);
+              ld4(zv + ij, z4);
+              if (!first) ld4(pold + ij, p4);
 #pragma unroll
               for (int jj = 0; jj < 4; jj++) {
                 const T pl = first ? z4[jj] : fmat<T>(beta[jj], p4[jj], z4[jj]);
@@ -487,8 +478,8 @@ __global__ void __launch_bounds__(kMultiThreads, B <= 2 ? (sizeof(T) == 4 ? 4 : 
         for (int cc = 0; cc < B; cc++) {
           const long long i = at(row, cc);
           T z4[4], p4[4], pn[4];
-          ld4<false>(zv + i, z4);
-          if (!first) ld4<false>(pold + i, p4);
+          ld4(zv + i, z4);
+          if (!first) ld4(pold + i, p4);
 #pragma unroll
           for (int jj = 0; jj < 4; jj++) {
             pn[jj] = first ? z4[jj] : fmat<T>(beta[jj], p4[jj], z4[jj]);
@@ -499,8 +490,8 @@ __global__ void __launch_bounds__(kMultiThreads, B <= 2 ? (sizeof(T) == 4 ? 4 : 
           if (fold[0] || fold[1] || fold[2] || fold[3]) {
             double x4[4];
             T y4[4];
-            ld4<false>(xv + i, x4);
-            ld4<false>(yv + i, y4);
+            ld4(xv + i, x4);
+            ld4(yv + i, y4);
 #pragma unroll
             for (int jj = 0; jj < 4; jj++)
               if (fold[jj] && live[jj]) {
@@ -512,9 +503,14 @@ __global__ void __launch_bounds__(kMultiThreads, B <= 2 ? (sizeof(T) == 4 ? 4 : 
           }
         }
       }
+      k0 = k1;
+      len = len1;
+      cj = cj1;
+#pragma unroll
+      for (int e = 0; e < B2; e++) vv[e] = vv1[e];
     }
     reduce_write(pq, zero4);
-    if (!grid_sync(c, a.partials, true, s_tot, a.spin_limit, [&] {
+    if (!grid_sync<TH>(c, a.partials, true, s_tot, s_parts, a.spin_limit, [&] {
           if (threadIdx.x < K && !vc->done[threadIdx.x]) {
             const int kk = threadIdx.x;
             const double w = s_tot[0][kk];
@@ -548,11 +544,11 @@ __global__ void __launch_bounds__(kMultiThreads, B <= 2 ? (sizeof(T) == 4 ? 4 : 
         for (int cc = 0; cc < B; cc++) {
           const long long i = at(row, cc);
           T p4[4], q4[4], r4[4], y4[4], z4[4] = {T(0), T(0), T(0), T(0)};
-          ld4<false>(pnew + i, p4);
-          ld4<false>(qv + i, q4);
-          ld4<false>(rv + i, r4);
-          ld4<false>(yv + i, y4);
-          if (keep_z) ld4<false>(zv + i, z4);
+          ld4(pnew + i, p4);
+          ld4(qv + i, q4);
+          ld4(rv + i, r4);
+          ld4(yv + i, y4);
+          if (keep_z) ld4(zv + i, z4);
 #pragma unroll
           for (int j = 0; j < 4; j++) {
             y4[j] = lv[j] ? fmat<T>(alpha[j], p4[j], y4[j]) : y4[j];
@@ -587,7 +583,7 @@ __global__ void __launch_bounds__(kMultiThreads, B <= 2 ? (sizeof(T) == 4 ? 4 : 
       }
       reduce_write(v0, v1);
     }
-    if (!grid_sync(c, a.partials, true, s_tot, a.spin_limit, [&] {
+    if (!grid_sync<TH>(c, a.partials, true, s_tot, s_parts, a.spin_limit, [&] {
           int any_r = 0;
           if (threadIdx.x < K && !vc->done[threadIdx.x]) {
             const int kk = threadIdx.x;
@@ -627,7 +623,7 @@ __global__ void __launch_bounds__(kMultiThreads, B <= 2 ? (sizeof(T) == 4 ? 4 : 
         mine[j] = k < K && __ldcg(&c->refresh[k]) != 0;
       }
       refresh(mine);
-      if (!grid_sync(c, a.partials, true, s_tot, a.spin_limit, [&] {
+      if (!grid_sync<TH>(c, a.partials, true, s_tot, s_parts, a.spin_limit, [&] {
             if (threadIdx.x < K && vc->refresh[threadIdx.x]) {
               const int kk = threadIdx.x;
               const double rr = s_tot[0][kk], rz = s_tot[1][kk];
@@ -685,8 +681,8 @@ __global__ void __launch_bounds__(kMultiThreads, B <= 2 ? (sizeof(T) == 4 ? 4 : 
         const long long i = at(row, cc);
         double x4[4];
         T y4[4];
-        ld4<false>(xv + i, x4);
-        ld4<false>(yv + i, y4);
+        ld4(xv + i, x4);
+        ld4(yv + i, y4);
 #pragma unroll
         for (int j = 0; j < 4; j++)
           if (fold[j]) {
@@ -739,24 +735,26 @@ cudaError_t grow_m(P** p, size_t& cap, size_t need) {
 // The chunk's work as one CUDA graph: right-hand sides to the interleaved
 // layout, control block cleared, the persistent kernel (cooperative launch:
 // every block resident), solutions back to the caller's layout.
-template <int B, class T, int Q>
+template <int B, class T, int Q, bool kStride>
 int capture_multi(const MultiArgs<T>& args, const double* d_B, double* b_dst, double* d_X, long long ld, int Kc,
                   cudaStream_t s, cudaGraph_t* graph) {
-  auto kernel = multi_cg_kernel<B, T, Q>;
+  auto kernel = multi_cg_kernel<B, T, Q, kStride>;
   constexpr int Kp = 4 * Q;
   int per_sm = 0, dev = 0, sms = 0;
-  MB_CUDA_OK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kMultiThreads, 0));
+  constexpr int TH = MultiShape<B, T, kStride>::threads;
+  MB_CUDA_OK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, TH, 0));
   MB_CUDA_OK(cudaGetDevice(&dev));
   MB_CUDA_OK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   if (per_sm < 1) return kBadInput;
-  // every block resident (cooperative launch), within the barrier's group table
-  const int grid = std::min(per_sm * sms, kMaxGroups * kBarrierGroup);
+  // every block resident (cooperative launch); a small system takes blocks
+  // with at least eight warps' rows each
+  const int grid = (int)std::max<long long>(1, std::min<long long>(std::min(per_sm, 2048 / TH) * sms, (args.N + 256 / Q - 1) / (256 / Q)));
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeCooperative;
   attr[0].val.cooperative = 1;
   cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(kMultiThreads);
+  cfg.blockDim = dim3(TH);
   cfg.stream = s;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
@@ -854,11 +852,14 @@ int multi_solve(SellMatrix& m, MultiState& ms, long long build_id, int n_rhs, co
   int dev = 0, sms = 0;
   MB_CUDA_OK(cudaGetDevice(&dev));
   MB_CUDA_OK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  // resident blocks x partials, then one row of group sums per group
-  const size_t part = ((size_t)sms * (2048 / kMultiThreads) + kMaxGroups) * 2 * kMultiK;
+  const size_t part = (size_t)sms * (2048 / 256) * 2 * kMultiK;  // every resident block's sums
   MB_CUDA_OK(grow_m(&ms.partials, ms.cap_part, part));
   if (!ms.ctl) MB_CUDA_OK(cudaMalloc((void**)&ms.ctl, sizeof(MultiCtl)));
   std::vector<MultiCtl> h(1);
+  // a run of rows to each block while an iteration's vectors stay in L2 (its
+  // gathers then find neighbours in L1); beyond, rows dealt in turn, so that
+  // all blocks stream one front of each vector
+  const bool stride = 6.0 * (double)ld * std::min(kMultiK, n_rhs) * (double)tsize > 128e6;
   for (int k0 = 0; k0 < n_rhs; k0 += kMultiK) {
     const int Kc = std::min(kMultiK, n_rhs - k0);
     const int Q = Kc <= 8 ? 2 : 8;  // lanes per row; right-hand sides padded to 4Q
@@ -873,6 +874,7 @@ int multi_solve(SellMatrix& m, MultiState& ms, long long build_id, int n_rhs, co
       append_bytes(key, Bn);
       append_bytes(key, Q);
       append_bytes(key, precision);
+      append_bytes(key, stride);
       append_bytes(key, Bk);
       append_bytes(key, Xk);
       append_bytes(key, ld);
@@ -890,8 +892,11 @@ int multi_solve(SellMatrix& m, MultiState& ms, long long build_id, int n_rhs, co
         append_bytes(key, a);
         for (auto& g : ms.graphs)
           if (g.key == key) return kOk;
-        return Q == 2 ? capture_multi<Bn, float, 2>(a, Bk, ms.b, Xk, ld, Kc, s, &graph)
-                      : capture_multi<Bn, float, 8>(a, Bk, ms.b, Xk, ld, Kc, s, &graph);
+        if (stride)
+          return Q == 2 ? capture_multi<Bn, float, 2, true>(a, Bk, ms.b, Xk, ld, Kc, s, &graph)
+                        : capture_multi<Bn, float, 8, true>(a, Bk, ms.b, Xk, ld, Kc, s, &graph);
+        return Q == 2 ? capture_multi<Bn, float, 2, false>(a, Bk, ms.b, Xk, ld, Kc, s, &graph)
+                      : capture_multi<Bn, float, 8, false>(a, Bk, ms.b, Xk, ld, Kc, s, &graph);
       }
       MultiArgs<double> a;
       memset(&a, 0, sizeof(a));
@@ -904,8 +909,11 @@ int multi_solve(SellMatrix& m, MultiState& ms, long long build_id, int n_rhs, co
       append_bytes(key, a);
       for (auto& g : ms.graphs)
         if (g.key == key) return kOk;
-      return Q == 2 ? capture_multi<Bn, double, 2>(a, Bk, ms.b, Xk, ld, Kc, s, &graph)
-                    : capture_multi<Bn, double, 8>(a, Bk, ms.b, Xk, ld, Kc, s, &graph);
+      if (stride)
+        return Q == 2 ? capture_multi<Bn, double, 2, true>(a, Bk, ms.b, Xk, ld, Kc, s, &graph)
+                      : capture_multi<Bn, double, 8, true>(a, Bk, ms.b, Xk, ld, Kc, s, &graph);
+      return Q == 2 ? capture_multi<Bn, double, 2, false>(a, Bk, ms.b, Xk, ld, Kc, s, &graph)
+                    : capture_multi<Bn, double, 8, false>(a, Bk, ms.b, Xk, ld, Kc, s, &graph);
     });
     if (rc) return rc;
     cudaGraphExec_t exec = nullptr;
