@@ -1087,7 +1087,8 @@ size_t persist_work_bytes(const SellMatrix& m, const SolveParams& p) {
 // scalars (same bits in every solve compared).
 bool persist_applies(const SellMatrix& m, const SolveParams& p) {
   const bool mixed = p.precision == 1;
-  if (p.shard || p.timers || (p.method != 1 && (p.method != 5 || mixed))) return false;
+  // (a matrix with columns beyond its rows has no place in the windows)
+  if (p.shard || p.np_rows != m.N || p.timers || (p.method != 1 && (p.method != 5 || mixed))) return false;
   const PersistPlan q = make_plan(m, p);
   double limit;  // MB
   if (p.method == 5) limit = m.ndof == 1 ? 32 : 100;
