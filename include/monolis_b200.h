@@ -44,15 +44,18 @@ static const int MONOLIS_B200_PRM_I_REFRESH_PERIOD = 41; /* mixed precision: FP6
 static const int MONOLIS_B200_PRM_I_WIDE_SLICES_FP64 = 42; /* out: 32-row slices that keep 32-bit column ids (the
                                                               others store 16-bit differences to a base per slot) */
 static const int MONOLIS_B200_PRM_I_WIDE_SLICES_FP32 = 43; /* out: same for the 64-row slices of the FP32 layout */
-static const int MONOLIS_B200_PRM_I_WAIT_LIMIT     = 44; /* many right-hand sides and one-kernel solves: polls after which a grid-barrier
-                                                            wait gives up and the solve returns MONOLIS_B200_TIMEOUT
-                                                            (0: 4,194,304, seconds) */
-static const int MONOLIS_B200_PRM_I_WAIT_DELAY_US  = 45; /* testing that bound: block 0 of the
-                                                            kernel reaches its first barrier this many microseconds
-                                                            late (0: off; at most 1,000,000) */
+static const int MONOLIS_B200_PRM_I_WAIT_LIMIT     = 44; /* many right-hand sides and one-kernel solves: polls after
+                                                            which a grid-wide wait gives up and the solve returns
+                                                            MONOLIS_B200_TIMEOUT, x partly written (0: 4,194,304,
+                                                            seconds) */
+static const int MONOLIS_B200_PRM_I_WAIT_DELAY_US  = 45; /* testing that bound: block 0 of the kernel reaches its first
+                                                            grid-wide wait this many microseconds late (0: off; at
+                                                            most 1,000,000) */
 static const int MONOLIS_B200_PRM_I_UNIFORM_SLICES_FP64 = 46; /* out: 32-row slices whose block columns are the
                                                             per-slot base plus the lane (no column stream read) */
 static const int MONOLIS_B200_PRM_I_UNIFORM_SLICES_FP32 = 47; /* out: same for the 64-row slices of the FP32 layout */
+static const int MONOLIS_B200_PRM_I_WAIT_DELAY_AT  = 48; /* WAIT_DELAY_US of one-kernel solves: the number of the wait
+                                                            that block 0 reaches late (0: the first) */
 
 static const int MONOLIS_B200_PRM_R_REFRESH_DELTA  = 30; /* mixed precision: FP64 refresh when ||r|| has dropped
                                                             below delta * its largest value since the last one

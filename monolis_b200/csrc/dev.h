@@ -220,7 +220,8 @@ struct SolveParams {
   const ShardPlan* shard = nullptr;  // multi-rank solve (FP64 CG); x holds np_rows block rows (ghosts last)
   int np_rows = 0;
   unsigned long long wait_limit = 0;  // one-kernel solves: polls before a grid-wide wait gives up (0: the default, seconds)
-  unsigned int delay_ns = 0;          // testing that bound: block 0 starts that much later
+  unsigned int delay_ns = 0;          // testing that bound: block 0 comes that much late ...
+  unsigned long long delay_at = 0;    // ... to its wait of this number (0: the first)
 };
 struct SolveResult {
   int iter = 0, status = 0, n_refine = 0;
@@ -237,7 +238,7 @@ int solve_device(SellMatrix& m, Scratch& sc, const SolveParams& p, const double*
 // ---- one-kernel solves (persist.cu) ----
 // persist_applies: the rule by which solve_device takes them. work:
 // persist_work_bytes() of device memory. The verdict is left in *st (not done
-// if a wait gave up).
+// if any block's wait gave up: x is then only partly written).
 bool persist_applies(const SellMatrix& m, const SolveParams& p);
 size_t persist_work_bytes(const SellMatrix& m, const SolveParams& p);
 int persist_solve(const SellMatrix& m, const SolveParams& p, const double* b, double* x, void* work, SolverState* st,

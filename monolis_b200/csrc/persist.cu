@@ -36,6 +36,7 @@ constexpr int kMaxWords = 4;     // two double-double sums
 struct ExchangeSlots {
   double w[2][kMaxWords][kMaxBlocks];
   unsigned long long arrived;
+  unsigned int finished;  // blocks that have written their part of X
 };
 struct ExchangeShared {
   double warp[32][kMaxWords];  // partial sums of this block's warps
@@ -43,7 +44,9 @@ struct ExchangeShared {
 };
 struct Exchange {
   ExchangeSlots* slots;
-  unsigned long long limit;  // polls before a wait gives up
+  unsigned long long limit;     // polls before a wait gives up
+  unsigned long long delay_at;  // testing that: block 0 arrives delay_ns late where target is this (0: nowhere)
+  unsigned int delay_ns;
   unsigned long long target = 0;
   int parity = 0;
 };
@@ -119,6 +122,8 @@ struct AccWords<DDAcc<K>> {
 // threads have met at a block barrier) is visible to every block that passes.
 __device__ __forceinline__ bool arrive_and_wait(Exchange& x) {
   unsigned long long v, n = 0;
+  if (x.target == x.delay_at && blockIdx.x == 0)
+    for (unsigned int t = 0; t < x.delay_ns; t += 1000) __nanosleep(1000);
   fence_gpu();
   asm volatile("red.relaxed.gpu.global.add.u64 [%0], 1;" ::"l"(&x.slots->arrived) : "memory");
   bool ok = true;
@@ -141,8 +146,10 @@ __device__ __forceinline__ bool arrive_and_wait(Exchange& x) {
 // result has to be sent back. On B200, 148 blocks: 3500 cycles (1.85 us) for
 // store, arrival, wait and reading back; polling the blocks' slots instead of
 // a counter took 5800 (the pollers delay the stores), pushing the sums to
-// every block 4900. A wait is bounded; false (in every thread) once one has
-// run out.
+// every block 4900. A wait is bounded; false (in every thread) where this
+// block's has run out. It has arrived all the same, so blocks that come later
+// pass and only miss it at the next exchange: after the last one they end the
+// solve without it, which is why the verdict waits for `publish`.
 template <class A, class F>
 __device__ __forceinline__ bool grid_exchange(Exchange& x, ExchangeShared& sh, A v, F&& fin) {
   using W = AccWords<A>;
@@ -223,7 +230,7 @@ struct PersistArgs {
   SolverState* st;
   double* hist;
   ExchangeSlots* slots;
-  unsigned long long limit;
+  unsigned long long limit, delay_at;
   unsigned int delay_ns;
   int per;       // slices of a block, at most
   int win_rows;  // rows of a window, at most
@@ -684,11 +691,16 @@ __device__ __forceinline__ void residual(const PersistArgs<T>& a, const BlockRow
   }
 }
 
+// The end of a block that has written its part of X: the last of the grid
+// leaves the verdict (S has the same bits in every block). One that gave up a
+// wait never comes here, and *a.st then stays without a verdict.
 template <class T>
-__device__ __forceinline__ void start(const PersistArgs<T>& a, SolverState& S) {
-  if (threadIdx.x == 0) S = *a.st;
-  if (a.delay_ns && blockIdx.x == 0 && threadIdx.x == 0)
-    for (unsigned int t = 0; t < a.delay_ns; t += 1000) __nanosleep(1000);
+__device__ __forceinline__ void publish(const PersistArgs<T>& a, const SolverState& S) {
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    fence_gpu();
+    if (atomicAdd(&a.slots->finished, 1u) == gridDim.x - 1) *a.st = S;
+  }
 }
 
 // dst = src on the block's entries
@@ -705,8 +717,8 @@ __global__ void __launch_bounds__(TH, 1) persist_cg_kernel(const PersistArgs<T> 
   constexpr bool kMixed = sizeof(T) == 4;
   __shared__ SolverState S;
   __shared__ ExchangeShared sh;
-  Exchange ex{a.slots, a.limit};
-  start(a, S);
+  Exchange ex{a.slots, a.limit, a.delay_at, a.delay_ns};
+  if (threadIdx.x == 0) S = *a.st;
   BlockRows<T> m = block_rows<B, kWin>(a);
   T* r = own_vector<B>(a, m, 0);
   T* q = own_vector<B>(a, m, 1);
@@ -837,7 +849,7 @@ __global__ void __launch_bounds__(TH, 1) persist_cg_kernel(const PersistArgs<T> 
   } else {
     copy_own<B, T>(m, xg, xo);
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) *a.st = S;
+  publish(a, S);
 }
 
 // ---------------------------------------------------------------------------
@@ -848,8 +860,8 @@ __global__ void __launch_bounds__(TH, 1) persist_bicg_kernel(const PersistArgs<d
   using T = double;
   __shared__ SolverState S;
   __shared__ ExchangeShared sh;
-  Exchange ex{a.slots, a.limit};
-  start(a, S);
+  Exchange ex{a.slots, a.limit, a.delay_at, a.delay_ns};
+  if (threadIdx.x == 0) S = *a.st;
   BlockRows<T> m = block_rows<B, false>(a);
   T* r = own_vector<B>(a, m, 0);
   T* vv = own_vector<B>(a, m, 1);
@@ -1002,7 +1014,7 @@ __global__ void __launch_bounds__(TH, 1) persist_bicg_kernel(const PersistArgs<d
   }
   // the last exchange is behind: no block reads X any more
   copy_own<B, T>(m, a.x, xo);
-  if (blockIdx.x == 0 && threadIdx.x == 0) *a.st = S;
+  publish(a, S);
 }
 
 // Threads of a block, slots of a chunk and chunk buffers, by block size.
@@ -1124,6 +1136,7 @@ int persist_solve(const SellMatrix& m, const SolveParams& p, const double* b, do
     a.hist = hist;
     a.slots = (ExchangeSlots*)work;
     a.limit = p.wait_limit ? p.wait_limit : 1ull << 22;
+    a.delay_at = p.delay_ns ? (p.delay_at + 1) * (unsigned long long)q.grid : 0;
     a.delay_ns = p.delay_ns;
     a.per = q.per;
     a.win_rows = q.win_rows;

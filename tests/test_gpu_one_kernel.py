@@ -150,3 +150,40 @@ def test_one_kernel_wait_runs_out(gpu, method):
     rc, x, it = device_solve(m, b, False)
     rc0, x0, it0 = device_solve(m, b, True)
     assert rc == rc0 and it == it0 and bits_equal(x, x0)
+
+
+@pytest.mark.parametrize("ndof,shuffle,method,precision", [
+    (1, False, api.ITER_CG, 0), (1, True, api.ITER_CG, 0), (4, False, api.ITER_CG, 0), (1, False, api.ITER_CG, 1),
+    (1, False, api.ITER_BICGSTAB, 0),
+])
+def test_one_kernel_any_wait_runs_out(gpu, ndof, shuffle, method, precision):
+    """Block 0 late at each wait of a solve in turn, the last one included
+    (where the other blocks have given up and left, and block 0 finds every sum
+    complete): always TIMEOUT, never a verdict over an x that some blocks have
+    not written. Late at a wait beyond the last, the solve is the plain one."""
+    index, item, val, b = grid_system((15, 14, 13), ndof, 5, shuffle, skew=0.3 if method == api.ITER_BICGSTAB else 0.0)
+    n = len(index) - 1
+    m = api.Monolis(gpu)
+    m.set_matrix_BCSR(n, n, ndof, len(item), val.reshape(-1), index, item)
+    m.quiet()
+    m.set_error_abort(False)
+    m.set_method(method)
+    m.set_precision(precision)
+    m.set_tolerance(1e-12)
+    m.set_maxiter(5)
+    m.Iarray[api.B200_PRM_I_ITER_RR] = 3
+    m.device_prepare()
+    plain = device_solve(m, b, False)
+    assert plain[0] == 1 and plain[2] == 5
+    m.Iarray[api.B200_PRM_I_WAIT_LIMIT] = 2000
+    m.Iarray[api.B200_PRM_I_WAIT_DELAY_US] = 20000
+    codes = []
+    for k in range(64):
+        m.Iarray[api.B200_PRM_I_WAIT_DELAY_AT] = k
+        rc, x, it = device_solve(m, b, False)
+        codes.append(rc)
+        if rc != 4:
+            break
+    assert codes[:-1] == [4] * (len(codes) - 1) and codes[-1] == 1, codes
+    assert len(codes) - 1 >= 2 * 5 + 1  # two waits an iteration at the least
+    assert it == 5 and bits_equal(x, plain[1])
