@@ -236,7 +236,10 @@ double monolis_b200_batch_last_seconds(monolis_b200_batch* batch);
  *     (d_scale ? d_scale[e] : 1) * d_val[e*val_stride + k] (row-major
  *     (n_base*ndof)^2, val_stride 0: one shared matrix), all device arrays;
  *   set_Dirichlet: n_bc conditions (host lists node_id, n_dof_bc, val, in
- *     call order), d_b the device right-hand side updated in place. */
+ *     call order), d_b the device right-hand side updated in place.
+ * A refused call (BAD_INPUT: a node out of range, an element entry outside
+ * the pattern, a condition on a row without diagonal block) leaves the values
+ * and d_b as they were. */
 int monolis_b200_device_clear_matrix(MONOLIS* mat);
 int monolis_b200_device_add_elements_R(MONOLIS* mat, int n_elem, int n_base, const int* d_elem, const double* d_val,
                                        long long val_stride, const double* d_scale);

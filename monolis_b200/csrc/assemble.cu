@@ -278,12 +278,18 @@ __global__ void __launch_bounds__(256) add_elements_kernel(const int* __restrict
   if (lane == 0 && got != want) atomicOr(bad, 2);
 }
 
-// first and last condition of every dof (ord, last: their positions in the list)
-__global__ void dirichlet_list_kernel(const long long* __restrict__ dof, int n_bc, int* __restrict__ ord,
-                                      int* __restrict__ last) {
+// first and last condition of every dof (ord, last: their positions in the
+// list); bad: a fixed dof's row has no diagonal block
+__global__ void dirichlet_list_kernel(const long long* __restrict__ dof, int n_bc, const int* __restrict__ rowptr,
+                                      const int* __restrict__ item, int ndof, int* __restrict__ ord,
+                                      int* __restrict__ last, int* __restrict__ bad) {
   for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n_bc; q += gridDim.x * blockDim.x) {
     atomicMin(reinterpret_cast<unsigned int*>(ord) + dof[q], (unsigned int)q);
     atomicMax(last + dof[q], q);
+    const int i = (int)(dof[q] / ndof);
+    bool diag = find_slot(rowptr, item, i, i) >= 0;
+    for (int k = rowptr[i]; !diag && k < rowptr[i + 1]; k++) diag = item[k] - 1 == i;  // a row not in order
+    if (!diag) atomicOr(bad, 1);
   }
 }
 
@@ -291,18 +297,19 @@ __global__ void dirichlet_list_kernel(const long long* __restrict__ dof, int n_b
 // over the fixed columns c of the row in the order of their first occurrence
 // (never-fixed dofs n), then zero fixed rows and columns, unit diagonal of
 // fixed dofs, b = last value, in the CSR values and in the sliced layout. A
-// row that touches no fixed dof reads its columns and their marks only.
+// row that touches no fixed dof reads its columns and their marks only. Bad
+// conditions leave everything as it was.
 template <int B>
 __global__ void __launch_bounds__(256) dirichlet_kernel(const int* __restrict__ rowptr, const int* __restrict__ item,
                                                         int N, double* __restrict__ A, const long long* __restrict__ slptr,
                                                         double* __restrict__ sell, const int* __restrict__ ord,
                                                         const int* __restrict__ last, const double* __restrict__ val,
-                                                        double* __restrict__ b, int* __restrict__ bad) {
+                                                        double* __restrict__ b, const int* __restrict__ bad) {
   constexpr int B2 = B * B;
   constexpr unsigned kAll = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const int i = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-  if (i >= N) return;  // whole warps
+  if (i >= N || *bad) return;  // whole warps
   const int lo = rowptr[i], hi = rowptr[i + 1];
   bool fr[B], own = false;
 #pragma unroll
@@ -353,10 +360,8 @@ __global__ void __launch_bounds__(256) dirichlet_kernel(const int* __restrict__ 
   }
   __syncwarp();
   const long long base = slptr[i >> 5];
-  bool diag = false;
   for (int k = lo + lane; k < hi; k += 32) {
     const long long j = item[k] - 1;
-    diag |= j == i;
     double* dst = A + (long long)k * B2;
     double* sl = sell + (base + (long long)(k - lo) * kSlice) * B2 + (i & (kSlice - 1));
 #pragma unroll
@@ -371,12 +376,10 @@ __global__ void __launch_bounds__(256) dirichlet_kernel(const int* __restrict__ 
         }
     }
   }
-  diag = __any_sync(kAll, diag);
   if (lane == 0) {
 #pragma unroll
     for (int r = 0; r < B; r++)
       if (fr[r]) b[(long long)i * B + r] = val[last[(long long)i * B + r]];
-    if (own && !diag) atomicOr(bad, 4);
   }
 }
 
@@ -439,18 +442,24 @@ int device_add_elements(SellMatrix& m, int NP, int n_elem, int n_base, const int
   if (rc) return rc;
   MB_CUDA_OK(cudaGetLastError());
   const bool had[3] = {m.have_val32, m.have_alu, m.have_alu32};
-  rc = sell_refill(m, s);
+  rc = sell_refill(m, s, d_bad);
   if (rc) return rc;
   int bad = 0;
   MB_CUDA_OK(cudaMemcpyAsync(&bad, d_bad, sizeof(int), cudaMemcpyDeviceToHost, s));
   MB_CUDA_OK(cudaStreamSynchronize(s));
-  if (bad & 1) {  // nothing has been added
-    m.have_val32 = had[0];
-    m.have_alu = had[1];
-    m.have_alu32 = had[2];
+  if (!bad) return kOk;
+  // refused: the layout has not been refilled, and what is derived from it stands
+  m.have_val32 = had[0];
+  m.have_alu = had[1];
+  m.have_alu32 = had[2];
+  if (bad & 2) {
+    // the entries that are in the pattern have been added: back to the layout's values
+    fprintf(stderr, "** monolis_b200: device assembly: an element entry is not in the nonzero pattern\n");
+    rc = sell_restore_csr(m, s);
+    if (rc) return rc;
+    MB_CUDA_OK(cudaStreamSynchronize(s));
   }
-  if (bad & 2) fprintf(stderr, "** monolis_b200: device assembly: an element entry is not in the nonzero pattern\n");
-  return bad ? kBadInput : kOk;
+  return kBadInput;
 }
 
 int device_dirichlet(SellMatrix& m, double* d_b, int n_bc, const int* node, const int* dof, const double* val,
@@ -477,7 +486,8 @@ int device_dirichlet(SellMatrix& m, double* d_b, int n_bc, const int* node, cons
   MB_CUDA_OK(cudaMemsetAsync(d_bad, 0, sizeof(int), s));
   MB_CUDA_OK(cudaMemcpyAsync(d_dof, flat.data(), sizeof(long long) * n_bc, cudaMemcpyHostToDevice, s));
   MB_CUDA_OK(cudaMemcpyAsync(d_val, val, sizeof(double) * n_bc, cudaMemcpyHostToDevice, s));
-  dirichlet_list_kernel<<<std::min((n_bc + 255) / 256, 148 * 8), 256, 0, s>>>(d_dof, n_bc, d_ord, d_last);
+  dirichlet_list_kernel<<<std::min((n_bc + 255) / 256, 148 * 8), 256, 0, s>>>(d_dof, n_bc, m.d_rowptr, m.d_item, nd,
+                                                                           d_ord, d_last, d_bad);
   int rc = dispatch_ndof(nd, [&](auto Bc) {
     constexpr int B = decltype(Bc)::value;
     dirichlet_kernel<B><<<warps_grid(N), 256, 0, s>>>(m.d_rowptr, m.d_item, N, m.d_csrval, m.d_slptr, m.d_val64, d_ord,
@@ -486,7 +496,6 @@ int device_dirichlet(SellMatrix& m, double* d_b, int n_bc, const int* node, cons
   });
   if (rc) return rc;
   MB_CUDA_OK(cudaGetLastError());
-  sell_values_changed(m);
   int bad = 0;
   MB_CUDA_OK(cudaMemcpyAsync(&bad, d_bad, sizeof(int), cudaMemcpyDeviceToHost, s));
   MB_CUDA_OK(cudaStreamSynchronize(s));
@@ -494,6 +503,7 @@ int device_dirichlet(SellMatrix& m, double* d_b, int n_bc, const int* node, cons
     fprintf(stderr, "** monolis_b200: set Dirichlet: diagonal block not found\n");
     return kBadInput;
   }
+  sell_values_changed(m);
   return kOk;
 }
 

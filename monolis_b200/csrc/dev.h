@@ -130,8 +130,11 @@ int sell_build(SellMatrix& m, const int* h_index, const int* h_item, const doubl
 // Slices and FP64 values from the device CSR (d_rowptr, d_item, d_csrval).
 int sell_layout(SellMatrix& m, cudaStream_t s);
 // The device CSR values have changed, the pattern has not: FP64 values of the
-// layout again (the FP32 copy and the DIAG factors follow on demand).
-int sell_refill(SellMatrix& m, cudaStream_t s);
+// layout again (the FP32 copy and the DIAG factors follow on demand); nothing
+// where the device word d_refused is set.
+int sell_refill(SellMatrix& m, cudaStream_t s, const int* d_refused = nullptr);
+// The device CSR values back to the layout's.
+int sell_restore_csr(SellMatrix& m, cudaStream_t s);
 void sell_values_changed(SellMatrix& m);  // drops the FP32 copy and the DIAG factors
 // A^T from A's device CSR and the host CSC arrays of the pattern (offsets,
 // 1-based rows, 1-based CSR positions; monolis_get_CSC_format).

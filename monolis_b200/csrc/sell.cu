@@ -74,15 +74,17 @@ __global__ void sell2_fill_kernel(const int* __restrict__ rowptr, const int* __r
 }
 
 // One warp per slice: lane l copies row (32s + l) into the slot-major layout
-// (kCols: column ids too; without, the values of an unchanged pattern only).
+// (kCols: column ids too; without, the values of an unchanged pattern only,
+// and nothing where *refused is set).
 template <int B, bool kCols>
 __global__ void sell_fill_kernel(const int* __restrict__ rowptr, const int* __restrict__ item,
                                  const double* __restrict__ csrval, const long long* __restrict__ slptr,
-                                 int N, int nslices, int* __restrict__ col, double* __restrict__ val) {
+                                 int N, int nslices, int* __restrict__ col, double* __restrict__ val,
+                                 const int* __restrict__ refused = nullptr) {
   constexpr int B2 = B * B;
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
-  if (warp >= nslices) return;
+  if (warp >= nslices || (refused && *refused)) return;
   const int row = warp * kSlice + lane;
   const long long base = slptr[warp];
   const int w = (int)((slptr[warp + 1] - base) / kSlice);
@@ -100,6 +102,23 @@ __global__ void sell_fill_kernel(const int* __restrict__ rowptr, const int* __re
       for (int e = 0; e < B2; e++) val[(slot * B2) + (long long)e * kSlice + lane] = 0.0;
     }
   }
+}
+
+// The inverse: the CSR values from the layout's.
+template <int B>
+__global__ void csr_fill_kernel(const int* __restrict__ rowptr, const long long* __restrict__ slptr, int N, int nslices,
+                                const double* __restrict__ val, double* __restrict__ csrval) {
+  constexpr int B2 = B * B;
+  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  const int row = warp * kSlice + lane;
+  if (warp >= nslices || row >= N) return;
+  const long long base = slptr[warp], j0 = rowptr[row];
+  const int len = rowptr[row + 1] - rowptr[row];
+  for (int k = 0; k < len; k++)
+#pragma unroll
+    for (int e = 0; e < B2; e++)
+      csrval[(j0 + k) * B2 + e] = val[(base + (long long)k * kSlice) * B2 + (long long)e * kSlice + lane];
 }
 
 // Compressed column ids of one layout, P rows per lane (P = 1: 32-row slices;
@@ -417,17 +436,29 @@ void sell_values_changed(SellMatrix& m) { m.have_val32 = m.have_alu = m.have_alu
 
 // The FP64 values again from the device CSR values; slices and columns stay
 // (padded slots keep their zeros).
-int sell_refill(SellMatrix& m, cudaStream_t s) {
+int sell_refill(SellMatrix& m, cudaStream_t s, const int* d_refused) {
   const unsigned blocks = (unsigned)(((long long)m.nslices * 32 + 255) / 256);
   int rc = dispatch_ndof(m.ndof, [&](auto Bc) {
     constexpr int B = decltype(Bc)::value;
     sell_fill_kernel<B, false><<<blocks, 256, 0, s>>>(m.d_rowptr, m.d_item, m.d_csrval, m.d_slptr, m.N, m.nslices,
-                                                      m.d_col, m.d_val64);
+                                                      m.d_col, m.d_val64, d_refused);
     return kOk;
   });
   if (rc) return rc;
   MB_CUDA_OK(cudaGetLastError());
   sell_values_changed(m);
+  return kOk;
+}
+
+int sell_restore_csr(SellMatrix& m, cudaStream_t s) {
+  const unsigned blocks = (unsigned)(((long long)m.nslices * 32 + 255) / 256);
+  int rc = dispatch_ndof(m.ndof, [&](auto Bc) {
+    constexpr int B = decltype(Bc)::value;
+    csr_fill_kernel<B><<<blocks, 256, 0, s>>>(m.d_rowptr, m.d_slptr, m.N, m.nslices, m.d_val64, m.d_csrval);
+    return kOk;
+  });
+  if (rc) return rc;
+  MB_CUDA_OK(cudaGetLastError());
   return kOk;
 }
 

@@ -126,3 +126,58 @@ def test_bad_elements_leave_the_values(gpu):
     assert gpu.monolis_b200_device_clear_matrix(m.p) == 0
     assert gpu.monolis_b200_device_add_elements_R(m.p, len(bad), 2, d_elem.data_ptr(), d_val.data_ptr(), 0, None) == 5
     assert not device_values(m, gpu).any()
+
+
+@pytest.mark.parametrize("ndof", [1, 3, 6])
+def test_refused_calls_change_nothing(gpu, ndof):
+    """An element entry outside the pattern (with others inside it) and a
+    condition on a row without diagonal block (after a good one): status 5, and
+    the values, the right-hand side, the FP64, FP32 and transposed products and
+    the DIAG factors stay what they were; the calls that follow work on them."""
+    import torch
+    n, rng = 75, np.random.default_rng(9)
+    cols = [[j for j in (i - 1, i, i + 1) if 0 <= j < n and not i == j == 40] for i in range(n)]
+    index = np.concatenate([[0], np.cumsum([len(c) for c in cols])]).astype(np.int32)
+    item = np.concatenate(cols).astype(np.int32)
+    val = rng.standard_normal(len(item) * ndof * ndof)
+    mh, m = api.Monolis(gpu), api.Monolis(gpu)
+    for q in (mh, m):
+        q.set_matrix_BCSR(n, n, ndof, len(item), val, index, item)
+        q.quiet()
+    m.set_precision(1)
+    m.set_matrix_cache(True)
+    m.device_prepare()
+    x = torch.from_numpy(rng.standard_normal(n * ndof)).cuda()
+    b = rng.standard_normal(n * ndof)
+    d_b = torch.from_numpy(b).cuda()
+
+    def state():
+        y, yt, y32 = torch.zeros_like(x), torch.zeros_like(x), torch.zeros(n * ndof, dtype=torch.float32, device="cuda")
+        x32 = x.float()
+        diag = np.empty(n * ndof * ndof)
+        torch.cuda.synchronize()
+        m.device_matvec(x.data_ptr(), y.data_ptr())
+        assert gpu.monolis_b200_device_matvec_R32(m.p, x32.data_ptr(), y32.data_ptr()) == 0
+        assert gpu.monolis_b200_device_matvec_transpose_R(m.p, x.data_ptr(), yt.data_ptr()) == 0
+        assert gpu.monolis_b200_device_get_diag(m.p, diag.ctypes.data_as(api._dp)) == 0
+        torch.cuda.synchronize()
+        return [a.cpu().numpy() for a in (y, yt, y32, d_b)] + [diag, device_values(m, gpu)]
+
+    def conditions(nodes, v):
+        nodes, dofs, v = np.array(nodes, dtype=np.int32), np.zeros(len(nodes), dtype=np.int32), np.array(v)
+        return gpu.monolis_b200_device_set_Dirichlet_bc_R(m.p, d_b.data_ptr(), len(nodes), nodes.ctypes.data_as(api._ip),
+                                                          dofs.ctypes.data_as(api._ip), v.ctypes.data_as(api._dp))
+
+    before = state()
+    elem = np.array([[3, 4], [20, 22], [60, 61]], dtype=np.int32)
+    ke = rng.standard_normal((2 * ndof) ** 2)
+    d_elem, d_ke = torch.from_numpy(elem).cuda(), torch.from_numpy(ke).cuda()
+    torch.cuda.synchronize()
+    assert gpu.monolis_b200_device_add_elements_R(m.p, 3, 2, d_elem.data_ptr(), d_ke.data_ptr(), 0, None) == 5
+    assert all(bits_equal(p, q) for p, q in zip(before, state()))
+    assert conditions([10, 40], [1.5, 2.5]) == 5
+    assert all(bits_equal(p, q) for p, q in zip(before, state()))
+    assert conditions([10, 74, 11], [1.5, -2.0, 0.5]) == 0
+    for node, v in ((10, 1.5), (74, -2.0), (11, 0.5)):
+        mh.set_Dirichlet_bc(b, node, 0, v)
+    assert bits_equal(device_values(m, gpu), mh.values()) and bits_equal(d_b.cpu().numpy(), b)
