@@ -39,18 +39,22 @@ constexpr int kMultiK = 32;
 // default bound of every barrier wait: polls of an L2 round trip, seconds in all
 constexpr unsigned long long kSpinLimit = 1ull << 22;
 
-// Threads of a block. Matrices of 1x1 and 2x2 blocks run one block to an SM, so
-// that an SM's rows are one run and the barrier has few arrivals: 768 threads
-// of 80 registers, or in FP32, where an iteration's vectors do not stay in L2
-// (kStride), 1024 of 64 (more loads in flight for HBM; they spill a little).
-// Larger blocks run as many blocks as fit. us an iteration, 768 / 1024
-// threads, 7-entry rows, FP32: 50^3 x 32 right-hand sides 78.8 / 81.7, 30^3 x 5
-// 30.0 / 34.7, 96^3 x 32 430 / 383; the form before (592 blocks of 256 threads,
-// a two-level barrier, gathers past L1, no prefetch) 83, 37 and 382, 12^3 x 32
-// 44 against 29; FP64 96^3 x 32 716 against 650.
+// Threads of a block, and whether the product loads a row's first blocks while
+// it works on the row before. Matrices of 1x1 and 2x2 blocks run one block to
+// an SM, so that an SM's rows are one run and the barrier has few arrivals; the
+// threads are what the registers allow without spilling much. 1x1: 768 of 80
+// registers, or in FP32, where an iteration's vectors do not stay in L2
+// (kStride), 1024 of 64 (more loads in flight for HBM). 2x2: 768 in FP32, 512
+// in FP64 (768 spill 800 bytes: 52^3 x 32 right-hand sides, 7-entry rows, 278
+// us an iteration against 230; 20^3 x 5 32.9 and 29.1). Larger blocks run as
+// many blocks of 256 as fit; the blocks loaded ahead spill 1.1 KB at 6x6 in
+// FP64 and 110 bytes at 5x5 (40^3 x 5: ndof 6 260 us an iteration with them,
+// 210 without; ndof 5 166 and 151) and are left out there.
 template <int B, class T, bool kStride>
 struct MultiShape {
-  static constexpr int threads = B > 2 ? 256 : (sizeof(T) == 4 && kStride ? 1024 : 768);
+  static constexpr bool fp32 = sizeof(T) == 4;
+  static constexpr int threads = B > 2 ? 256 : (B == 2 ? (fp32 ? 768 : 512) : (fp32 && kStride ? 1024 : 768));
+  static constexpr bool ahead = fp32 || B < 5;
 };
 
 struct MultiCtl {
@@ -187,6 +191,7 @@ __device__ __forceinline__ void st4(double* p, const double (&o)[4]) {
 template <int B, class T, int Q, bool kStride>
 __global__ void __launch_bounds__(MultiShape<B, T, kStride>::threads, 1) multi_cg_kernel(const MultiArgs<T> a) {
   constexpr int TH = MultiShape<B, T, kStride>::threads;
+  constexpr bool kAhead = MultiShape<B, T, kStride>::ahead;
   constexpr int B2 = B * B;
   constexpr int Kp = 4 * Q;
   constexpr int RPW = 32 / Q;  // rows per warp
@@ -419,8 +424,8 @@ __global__ void __launch_bounds__(MultiShape<B, T, kStride>::threads, 1) multi_c
     // P = Z + beta P (own rows, to pnew); Q = A P with the neighbours' P
     // recomputed from Z and the old P; <P,Q>
     double pq[4] = {0.0, 0.0, 0.0, 0.0}, zero4[4] = {0.0, 0.0, 0.0, 0.0};
-    // the next rows' extent and first blocks are loaded ahead, so that a row
-    // waits for its gathers only
+    // the next rows' extent and (kAhead) first blocks are loaded ahead, so that
+    // a row waits for its gathers only
     int k0 = 0, len = 0, cj = 0;
     T vv[B2];
     auto extent = [&](long long row, int& k, int& l) {
@@ -434,14 +439,14 @@ __global__ void __launch_bounds__(MultiShape<B, T, kStride>::threads, 1) multi_c
       for (int e = 0; e < B2; e++) v[e] = has ? val[(long long)(k + qd) * B2 + e] : T(0);
     };
     extent(wrow0 + g, k0, len);
-    blocks(k0, len, cj, vv);
+    if constexpr (kAhead) blocks(k0, len, cj, vv);
     for (long long rb = wrow0; rb < N; rb += sweep) {
       const long long row = rb + g;
       const bool valid = row < N;
-      int k1, len1, cj1;
+      int k1, len1, cj1 = 0;
       T vv1[B2];
       extent(row + sweep, k1, len1);
-      blocks(k1, len1, cj1, vv1);
+      if constexpr (kAhead) blocks(k1, len1, cj1, vv1);
       const int mlen = warp_max(len);
       T acc[B][4];
 #pragma unroll
@@ -449,7 +454,7 @@ __global__ void __launch_bounds__(MultiShape<B, T, kStride>::threads, 1) multi_c
 #pragma unroll
         for (int j = 0; j < 4; j++) acc[cc][j] = T(0);
       for (int base = 0; base < mlen; base += Q) {
-        if (base) blocks(k0 + base, len - base, cj, vv);
+        if (base || !kAhead) blocks(k0 + base, len - base, cj, vv);
 #pragma unroll
         for (int u = 0; u < Q; u++) {
           const int j = __shfl_sync(0xffffffffu, cj, u, Q);
@@ -505,9 +510,11 @@ __global__ void __launch_bounds__(MultiShape<B, T, kStride>::threads, 1) multi_c
       }
       k0 = k1;
       len = len1;
-      cj = cj1;
+      if constexpr (kAhead) {
+        cj = cj1;
 #pragma unroll
-      for (int e = 0; e < B2; e++) vv[e] = vv1[e];
+        for (int e = 0; e < B2; e++) vv[e] = vv1[e];
+      }
     }
     reduce_write(pq, zero4);
     if (!grid_sync<TH>(c, a.partials, true, s_tot, s_parts, a.spin_limit, [&] {

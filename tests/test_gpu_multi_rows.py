@@ -11,6 +11,7 @@ import pytest
 from monolis_b200 import api
 from monolis_b200 import problems as P
 from helpers import build
+from test_gpu_one_kernel import grid_system
 
 pytestmark = pytest.mark.gpu
 
@@ -52,3 +53,24 @@ def test_multi_beyond_l2(gpu, precision):
     assert np.all(st == 0) and np.all(res < 1e-8)
     for k in (0, 13, 31):
         assert np.linalg.norm(B[k] - P.csr_matvec(index, item, val, X[k])) / np.linalg.norm(B[k]) < 1.01e-8, k
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("ndof,n_rhs", [(1, 29), (2, 6), (2, 13), (4, 23), (5, 8), (5, 31), (6, 3), (6, 25)])
+def test_multi_block_sizes(gpu, ndof, n_rhs, precision):
+    index, item, val, _ = grid_system((13, 9, 8), ndof, 21)
+    n = len(index) - 1
+    m = api.Monolis(gpu)
+    m.set_matrix_BCSR(n, n, ndof, len(item), val.reshape(-1), index, item)
+    m.quiet()
+    m.set_error_abort(False)
+    m.set_method(api.ITER_CG)
+    m.set_precond(api.PREC_DIAG)
+    m.set_tolerance(1e-8)
+    m.set_maxiter(2000)
+    m.set_precision(precision)
+    B = np.stack([P.uniform(90 + k, n * ndof) for k in range(n_rhs)])
+    X, its, res, st = m.solve_multi(B)
+    assert np.all(st == 0) and np.all(res < 1e-8)
+    for k in range(n_rhs):
+        assert np.linalg.norm(B[k] - m.matvec(X[k])) / np.linalg.norm(B[k]) < 1.01e-8, k
