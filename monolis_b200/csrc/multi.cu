@@ -863,13 +863,17 @@ int multi_solve(SellMatrix& m, MultiState& ms, long long build_id, int n_rhs, co
   MB_CUDA_OK(grow_m(&ms.partials, ms.cap_part, part));
   if (!ms.ctl) MB_CUDA_OK(cudaMalloc((void**)&ms.ctl, sizeof(MultiCtl)));
   std::vector<MultiCtl> h(1);
-  // a run of rows to each block while an iteration's vectors stay in L2 (its
-  // gathers then find neighbours in L1); beyond, rows dealt in turn, so that
-  // all blocks stream one front of each vector
-  const bool stride = 6.0 * (double)ld * std::min(kMultiK, n_rhs) * (double)tsize > 128e6;
   for (int k0 = 0; k0 < n_rhs; k0 += kMultiK) {
     const int Kc = std::min(kMultiK, n_rhs - k0);
     const int Q = Kc <= 8 ? 2 : 8;  // lanes per row; right-hand sides padded to 4Q
+    // A run of rows to each block while an iteration's vectors, padding
+    // included, stay in L2 (its gathers then find neighbours in L1); beyond,
+    // rows dealt in turn, so that all blocks stream one front of each vector.
+    // us an iteration, runs / dealt: FP32, 1x1, 27-entry rows, 32 right-hand
+    // sides, 108 MB 151 / 146, 121 MB 174 / 154; 4x4, 7-entry rows, 16 of them
+    // padded to 32, 197 MB 298 / 249; FP64, 3x3, 101 MB 82 / 86, 27-entry rows,
+    // 124 MB 206 / 193
+    const bool stride = 6.0 * (double)ld * 4 * Q * (double)tsize > 105e6;
     const double* Bk = d_B + (long long)k0 * ld;
     double* Xk = d_X + (long long)k0 * ld;
     char* v = static_cast<char*>(ms.vec);
