@@ -95,16 +95,27 @@ __device__ __forceinline__ void st_release(unsigned int* p, unsigned int v) {
 
 __device__ __forceinline__ void fence_gpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
 
+// The scalars of the right-hand sides as of the last barrier, in the block's
+// shared memory. Every warp needs them after every barrier; read by every warp
+// from the control block, they made all SMs ask for the same two lines of L2 at
+// once, which cost 1 us a phase and four right-hand sides (20^3 x 28, FP64,
+// 7-entry rows 45 us an iteration; one warp of a block reading them 22).
+struct MultiScalars {
+  double alpha[kMultiK], beta[kMultiK];
+  int done[kMultiK], fold[kMultiK], refresh[kMultiK];
+  int it, any_refresh, all_done;
+};
+
 // Grid barrier of a cooperative launch, with an optional reduction of the
 // per-block partial sums (2 x 32 doubles per block, partials[block][64]): the
 // last block to arrive adds them, TH/64 strided parts of every sum and then the
 // parts in order, into tot and runs `last` (with all its threads) before
 // releasing everyone. One counter and one release word: 148 arrivals and
-// pollers are cheaper than a level of groups between. Waits are bounded;
-// returns false once any block has given up.
+// pollers are cheaper than a level of groups between. sc holds the scalars
+// afterwards. Waits are bounded; returns false once any block has given up.
 template <int TH, class F>
 __device__ bool grid_sync(MultiCtl* c, double* partials, bool reduce, double (*tot)[kMultiK], double* parts /* TH */,
-                          unsigned long long limit, F&& last) {
+                          unsigned long long limit, int K, MultiScalars& sc, F&& last) {
   __shared__ unsigned int s_gen;
   __shared__ int s_last, s_ok;
   const unsigned int G = gridDim.x;
@@ -149,7 +160,24 @@ __device__ bool grid_sync(MultiCtl* c, double* partials, bool reduce, double (*t
       }
     fence_gpu();
   }
-  if (threadIdx.x == 0) s_ok = __ldcg(&c->err) == 0;
+  if (threadIdx.x < kMultiK) {
+    __syncwarp();
+    const int k = threadIdx.x;
+    const int done = __ldcg(&c->done[k]), fold = __ldcg(&c->fold[k]), refresh = __ldcg(&c->refresh[k]);
+    const double alpha = __ldcg(&c->alpha[k]), beta = __ldcg(&c->beta[k]);
+    sc.done[k] = k >= K || done;
+    sc.fold[k] = k < K && fold;
+    sc.refresh[k] = k < K && refresh;
+    sc.alpha[k] = alpha;
+    sc.beta[k] = k < K ? beta : 0.0;
+    const int all = __all_sync(0xffffffffu, k >= K || done);
+    if (k == 0) {
+      s_ok = __ldcg(&c->err) == 0;
+      sc.it = __ldcg(&c->it);
+      sc.any_refresh = __ldcg(&c->any_refresh);
+      sc.all_done = all;
+    }
+  }
   __syncthreads();
   return s_ok != 0;
 }
@@ -210,7 +238,7 @@ __global__ void __launch_bounds__(MultiShape<B, T, kStride>::threads, 1) multi_c
   __shared__ double s_red[TH / 32][2][kMultiK];
   __shared__ double s_parts[TH];
   __shared__ double s_tot[2][kMultiK];
-  __shared__ int s_flag[2];
+  __shared__ MultiScalars sc;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const int qd = lane & (Q - 1);  // quad of right-hand sides
   const int g = lane / Q;         // row slot within the warp
@@ -222,7 +250,7 @@ __global__ void __launch_bounds__(MultiShape<B, T, kStride>::threads, 1) multi_c
   const int K = a.K;
   MultiCtl* c = a.ctl;
   // the last block of a barrier reads and writes the scalars through a
-  // volatile view (L1 is not coherent across SMs); the others use __ldcg
+  // volatile view (L1 is not coherent across SMs); the others use sc
   volatile MultiCtl* vc = c;
   auto at = [&](long long row, int comp) { return (row * B + comp) * Kp + 4 * qd; };
   auto warp_max = [](int v) {
@@ -260,10 +288,7 @@ __global__ void __launch_bounds__(MultiShape<B, T, kStride>::threads, 1) multi_c
   };
   auto live4 = [&](bool (&lv)[4]) {
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
-      const int k = 4 * qd + j;
-      lv[j] = k < K && __ldcg(&c->done[k]) == 0;
-    }
+    for (int j = 0; j < 4; j++) lv[j] = sc.done[4 * qd + j] == 0;
   };
 
   // x = y = 0 on the own rows
@@ -375,14 +400,14 @@ __global__ void __launch_bounds__(MultiShape<B, T, kStride>::threads, 1) multi_c
     for (unsigned int t = 0; t < a.delay_ns; t += 1000) __nanosleep(1000);
   }
   // the whole grid has zeroed its x and y before any residual reads them
-  if (!grid_sync<TH>(c, a.partials, false, s_tot, s_parts, a.spin_limit, [] {})) return;
+  if (!grid_sync<TH>(c, a.partials, false, s_tot, s_parts, a.spin_limit, K, sc, [] {})) return;
   {
     bool all[4];
 #pragma unroll
     for (int j = 0; j < 4; j++) all[j] = 4 * qd + j < K;
     refresh(all);
   }
-  if (!grid_sync<TH>(c, a.partials, true, s_tot, s_parts, a.spin_limit, [&] {
+  if (!grid_sync<TH>(c, a.partials, true, s_tot, s_parts, a.spin_limit, K, sc, [&] {
         if (threadIdx.x < kMultiK) {
           const int kk = threadIdx.x;
           const double rr = s_tot[0][kk], rz = s_tot[1][kk];
@@ -412,14 +437,14 @@ __global__ void __launch_bounds__(MultiShape<B, T, kStride>::threads, 1) multi_c
     bool live[4];
     live4(live);
     const bool any = live[0] || live[1] || live[2] || live[3];
-    const bool first = __ldcg(&c->it) == 1;
+    const bool first = sc.it == 1;
     T beta[4];
     bool fold[4];
 #pragma unroll
     for (int j = 0; j < 4; j++) {
       const int k = 4 * qd + j;
-      beta[j] = k < K ? (T)__ldcg(&c->beta[k]) : T(0);
-      fold[j] = k < K && __ldcg(&c->fold[k]) != 0;
+      beta[j] = (T)sc.beta[k];
+      fold[j] = sc.fold[k] != 0;
     }
     // P = Z + beta P (own rows, to pnew); Q = A P with the neighbours' P
     // recomputed from Z and the old P; <P,Q>
@@ -517,7 +542,7 @@ __global__ void __launch_bounds__(MultiShape<B, T, kStride>::threads, 1) multi_c
       }
     }
     reduce_write(pq, zero4);
-    if (!grid_sync<TH>(c, a.partials, true, s_tot, s_parts, a.spin_limit, [&] {
+    if (!grid_sync<TH>(c, a.partials, true, s_tot, s_parts, a.spin_limit, K, sc, [&] {
           if (threadIdx.x < K && !vc->done[threadIdx.x]) {
             const int kk = threadIdx.x;
             const double w = s_tot[0][kk];
@@ -538,7 +563,7 @@ __global__ void __launch_bounds__(MultiShape<B, T, kStride>::threads, 1) multi_c
       const bool anyl = lv[0] || lv[1] || lv[2] || lv[3];
       T alpha[4];
 #pragma unroll
-      for (int j = 0; j < 4; j++) alpha[j] = lv[j] ? (T)__ldcg(&c->alpha[4 * qd + j]) : T(0);
+      for (int j = 0; j < 4; j++) alpha[j] = lv[j] ? (T)sc.alpha[4 * qd + j] : T(0);
       double v0[4] = {0.0, 0.0, 0.0, 0.0}, v1[4] = {0.0, 0.0, 0.0, 0.0};
       // z is rewritten for the live right-hand sides; it is read only to keep
       // a stopped one's entries when this thread has one
@@ -590,7 +615,7 @@ __global__ void __launch_bounds__(MultiShape<B, T, kStride>::threads, 1) multi_c
       }
       reduce_write(v0, v1);
     }
-    if (!grid_sync<TH>(c, a.partials, true, s_tot, s_parts, a.spin_limit, [&] {
+    if (!grid_sync<TH>(c, a.partials, true, s_tot, s_parts, a.spin_limit, K, sc, [&] {
           int any_r = 0;
           if (threadIdx.x < K && !vc->done[threadIdx.x]) {
             const int kk = threadIdx.x;
@@ -622,15 +647,12 @@ __global__ void __launch_bounds__(MultiShape<B, T, kStride>::threads, 1) multi_c
           }
         }))
       return;
-    if (__ldcg(&c->any_refresh)) {
+    if (sc.any_refresh) {
       bool mine[4];
 #pragma unroll
-      for (int j = 0; j < 4; j++) {
-        const int k = 4 * qd + j;
-        mine[j] = k < K && __ldcg(&c->refresh[k]) != 0;
-      }
+      for (int j = 0; j < 4; j++) mine[j] = sc.refresh[4 * qd + j] != 0;
       refresh(mine);
-      if (!grid_sync<TH>(c, a.partials, true, s_tot, s_parts, a.spin_limit, [&] {
+      if (!grid_sync<TH>(c, a.partials, true, s_tot, s_parts, a.spin_limit, K, sc, [&] {
             if (threadIdx.x < K && vc->refresh[threadIdx.x]) {
               const int kk = threadIdx.x;
               const double rr = s_tot[0][kk], rz = s_tot[1][kk];
@@ -661,13 +683,7 @@ __global__ void __launch_bounds__(MultiShape<B, T, kStride>::threads, 1) multi_c
         return;
     }
     // every right-hand side done (or the iteration cap, as a backstop)
-    if (threadIdx.x == 0) {
-      int all = 1;
-      for (int kk = 0; kk < K; kk++) all &= __ldcg(&c->done[kk]) != 0;
-      s_flag[0] = all || __ldcg(&c->it) > a.max_iter + 1;
-    }
-    __syncthreads();
-    if (s_flag[0]) break;
+    if (sc.all_done || sc.it > a.max_iter + 1) break;
     T* tmp = pold;
     pold = pnew;
     pnew = tmp;
@@ -675,10 +691,7 @@ __global__ void __launch_bounds__(MultiShape<B, T, kStride>::threads, 1) multi_c
   // fold the last corrections (every block has passed its last reads of x, y)
   bool fold[4];
 #pragma unroll
-  for (int j = 0; j < 4; j++) {
-    const int k = 4 * qd + j;
-    fold[j] = k < K && __ldcg(&c->fold[k]) != 0;
-  }
+  for (int j = 0; j < 4; j++) fold[j] = sc.fold[4 * qd + j] != 0;
   if (fold[0] || fold[1] || fold[2] || fold[3])
     for (long long rb = wrow0; rb < N; rb += sweep) {
       const long long row = rb + g;
