@@ -1082,15 +1082,20 @@ size_t persist_work_bytes(const SellMatrix& m, const SolveParams& p) {
 // The one-kernel solve is taken while the matrix stream of an iteration (bytes
 // of the loop precision's layout) is small enough that the phases' launches
 // and reductions cost more than streaming from one block an SM with few loads
-// in flight does. us an iteration, kernel per phase / one kernel (B200, 27-
-// and 7-entry rows, 100 to 1200 iterations):
-//   CG, FP64, ndof 3        0.8 MB 31 / 12, 15 MB 28 / 12.4, 70 MB 35 / 19.4, 134 MB 42 / 34, 245 MB 64 / 61, 425 MB 92 / 93
-//   CG, refined, ndof 3     8 MB 28 / 11, 36 MB 30 / 14, 69 MB 34 / 21, 127 MB 42 / 36, 221 MB 57 / 53
-//   CG, FP64, ndof 1        0.1 MB 30 / 8.8, 11 MB 26 / 11, 24 MB 28 / 17, 47 MB 32 / 29, 60 MB 37 / 37, 140 MB 65 / 91
-//   CG, refined, ndof 1     7 MB 24 / 8.5, 30 MB 30 / 18, 37 MB 27 / 20, 58 MB 31 / 28, 84 MB 37 / 41
-//   CG, FP64, ndof 6        16 MB 37 / 19, 97 MB 48 / 41
-//   BiCGSTAB, FP64, ndof 1  1.2 MB 47 / 20, 29 MB 51 / 43, 60 MB 69 / 82
-//   BiCGSTAB, FP64, ndof 3  15 MB 47 / 32, 70 MB 60 / 49, 178 MB 120 / 122
+// in flight does. us an iteration, kernel per phase / one kernel (B200, solves
+// of 200 to 400 iterations; the stream in MB, 7- or 27-entry rows, grids in natural
+// and in random numbering and plates too wide for the window):
+//   CG, FP64      ndof 1  0.1 MB 30 / 8.8, 24 MB 28 / 16, no window: 47 MB 40 / 32, 50 MB 32 / 29
+//                 ndof 2  49 MB 39 / 27, 61 MB 36 / 33, 77 MB 39 / 39, 87 MB 42 / 44
+//                 ndof 3  0.8 MB 31 / 12, 134 MB 42 / 34, 218 MB 67 / 52, 245 MB 66 / 62; no window: 93 MB 46 / 33
+//                 ndof 4  93 MB 39 / 34;   ndof 5  94 MB 40 / 30;   ndof 6  82 MB 40 / 35, 90 MB 40 / 40
+//   CG, refined   ndof 1  7 MB 24 / 8.5, 50 MB 31 / 24; no window: 48 MB 46 / 37, 60 MB 35 / 34
+//                 ndof 2  56 MB 35 / 30, 79 MB 40 / 37, 84 MB 40 / 43
+//                 ndof 3  8 MB 28 / 11, 127 MB 42 / 36, 210 MB 60 / 51, 244 MB 66 / 67
+//                 ndof 4  91 MB 39 / 36;   ndof 5  93 MB 40 / 29;   ndof 6  91 MB 42 / 37
+//   BiCGSTAB      ndof 1  1.2 MB 47 / 20, 31 MB 49 / 40, 60 MB 69 / 82
+//                 ndof 2  47 MB 55 / 50, 61 MB 59 / 64;   ndof 3  63 MB 62 / 53, 76 MB 64 / 72 (random numbering 72 / 91)
+//                 ndof 4  93 MB 68 / 66;   ndof 5  94 MB 70 / 66;   ndof 6  82 MB 69 / 64, 90 MB 69 / 74
 // Refined BiCGSTAB stays with the kernels per phase: its dot products cancel,
 // so its FP32 recurrences hang on the grouping of their plain sums (symmetric
 // elasticity, 33^3 nodes: 1467 iterations with one, none within 20000 with
@@ -1102,10 +1107,11 @@ bool persist_applies(const SellMatrix& m, const SolveParams& p) {
   // (a matrix with columns beyond its rows has no place in the windows)
   if (p.shard || p.np_rows != m.N || p.timers || (p.method != 1 && (p.method != 5 || mixed))) return false;
   const PersistPlan q = make_plan(m, p);
-  double limit;  // MB
-  if (p.method == 5) limit = m.ndof == 1 ? 32 : 100;
-  else if (m.ndof == 1) limit = mixed ? 60 : 50;
-  else limit = q.window ? 250 : 100;
+  // MB by ndof; ndof 3 without a window: 100
+  static constexpr double kCg[6] = {50, 70, 250, 100, 100, 90}, kCgMixed[6] = {60, 80, 225, 100, 100, 100},
+                          kBicg[6] = {32, 52, 65, 95, 95, 80};
+  double limit = (p.method == 5 ? kBicg : mixed ? kCgMixed : kCg)[m.ndof - 1];
+  if (p.method == 1 && !q.window) limit = std::min(limit, 100.0);
   return q.ok && (mixed ? m.bytes32 : m.bytes64) <= limit * 1e6;
 }
 

@@ -187,3 +187,25 @@ def test_one_kernel_any_wait_runs_out(gpu, ndof, shuffle, method, precision):
     assert codes[:-1] == [4] * (len(codes) - 1) and codes[-1] == 1, codes
     assert len(codes) - 1 >= 2 * 5 + 1  # two waits an iteration at the least
     assert it == 5 and bits_equal(x, plain[1])
+
+
+@pytest.mark.parametrize("dims,ndof,method,precision,one", [
+    ((58, 58, 58), 2, api.ITER_CG, 0, True), ((66, 66, 66), 2, api.ITER_CG, 0, False),  # 52 and 76 MB
+    ((132, 132, 36), 2, api.ITER_CG, 1, False),  # 87 MB
+    ((55, 55, 55), 2, api.ITER_BICGSTAB, 0, True), ((62, 62, 62), 2, api.ITER_BICGSTAB, 0, False),  # 44 and 63 MB
+    ((52, 52, 52), 3, api.ITER_BICGSTAB, 0, False), ((35, 35, 36), 6, api.ITER_BICGSTAB, 0, False),  # 78 and 92 MB
+])
+def test_one_kernel_rule(gpu, dims, ndof, method, precision, one):
+    """One kernel up to the matrix stream at which the kernels per phase take over, by method and block size."""
+    index, item, val, b = grid_system(dims, ndof, 2)
+    n = len(index) - 1
+    m = api.Monolis(gpu)
+    m.set_matrix_BCSR(n, n, ndof, len(item), val.reshape(-1), index, item)
+    m.quiet()
+    m.set_error_abort(False)
+    m.set_method(method)
+    m.set_precision(precision)
+    m.set_maxiter(3)
+    m.device_prepare()
+    rc, x, it = device_solve(m, b, False)
+    assert rc == 1 and it == 3 and (m.Iarray[api.B200_PRM_I_LAUNCHES] == 1) == one
