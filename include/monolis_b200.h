@@ -56,6 +56,9 @@ static const int MONOLIS_B200_PRM_I_UNIFORM_SLICES_FP64 = 46; /* out: 32-row sli
 static const int MONOLIS_B200_PRM_I_UNIFORM_SLICES_FP32 = 47; /* out: same for the 64-row slices of the FP32 layout */
 static const int MONOLIS_B200_PRM_I_WAIT_DELAY_AT  = 48; /* WAIT_DELAY_US of one-kernel solves: the number of the wait
                                                             that block 0 reaches late (0: the first) */
+static const int MONOLIS_B200_PRM_I_REFUSE_LAUNCH  = 49; /* testing what follows when the device has no room for a
+                                                            one-kernel solve (a kernel per phase): 1 its launch, 2 its
+                                                            work memory is taken as refused (0: off) */
 
 static const int MONOLIS_B200_PRM_R_REFRESH_DELTA  = 30; /* mixed precision: FP64 refresh when ||r|| has dropped
                                                             below delta * its largest value since the last one

@@ -496,6 +496,7 @@ int solve_resident(MONOLIS* m, DevState* s, mb::SellMatrix& A, const double* d_b
   p.wait_limit = (unsigned long long)std::max(I[MONOLIS_B200_PRM_I_WAIT_LIMIT], 0);
   p.delay_ns = (unsigned int)std::min(std::max(I[MONOLIS_B200_PRM_I_WAIT_DELAY_US], 0), 1000000) * 1000u;
   p.delay_at = (unsigned long long)std::max(I[MONOLIS_B200_PRM_I_WAIT_DELAY_AT], 0);
+  p.refuse = I[MONOLIS_B200_PRM_I_REFUSE_LAUNCH];
   if (I[MONOLIS_PRM_I_SHOW_SUMMARY] == MONOLIS_I_TRUE)
     printf("** MONOLIS solver: %s, prec: %s\n", str_iter(p.method), str_prec(p.precond));
   const bool log = I[MONOLIS_PRM_I_SHOW_ITERLOG] == MONOLIS_I_TRUE;

@@ -225,6 +225,7 @@ struct SolveParams {
   unsigned long long wait_limit = 0;  // one-kernel solves: polls before a grid-wide wait gives up (0: the default, seconds)
   unsigned int delay_ns = 0;          // testing that bound: block 0 comes that much late ...
   unsigned long long delay_at = 0;    // ... to its wait of this number (0: the first)
+  int refuse = 0;  // testing the way back to the kernels per phase: 1 the launch, 2 the work memory is taken as refused
 };
 struct SolveResult {
   int iter = 0, status = 0, n_refine = 0;
@@ -243,6 +244,8 @@ int solve_device(SellMatrix& m, Scratch& sc, const SolveParams& p, const double*
 // persist_work_bytes() of device memory. The verdict is left in *st (not done
 // if any block's wait gave up: x is then only partly written).
 bool persist_applies(const SellMatrix& m, const SolveParams& p);
+// kRefused: the device did not take the launch and nothing has run.
+constexpr int kRefused = -1;
 size_t persist_work_bytes(const SellMatrix& m, const SolveParams& p);
 int persist_solve(const SellMatrix& m, const SolveParams& p, const double* b, double* x, void* work, SolverState* st,
                   double* hist, cudaStream_t s);

@@ -1149,7 +1149,8 @@ int persist_solve(const SellMatrix& m, const SolveParams& p, const double* b, do
     a.cb_cap = q.cb_cap;
     a.win_at = meta_bytes(q.per, q.cb_cap);
     a.smem = q.smem;
-    MB_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes) != cudaSuccess)
+      return kRefused;
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeCooperative;
@@ -1161,8 +1162,9 @@ int persist_solve(const SellMatrix& m, const SolveParams& p, const double* b, do
     cfg.stream = s;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    MB_CUDA_OK(cudaLaunchKernelEx(&cfg, kernel, a));
-    return kOk;
+    // a fault of an earlier kernel comes back here too, and again from the next call
+    const cudaError_t e = p.refuse == 1 ? cudaErrorCooperativeLaunchTooLarge : cudaLaunchKernelEx(&cfg, kernel, a);
+    return e == cudaSuccess ? kOk : kRefused;
   };
   return dispatch_ndof(m.ndof, [&](auto Bc) -> int {
     constexpr int B = decltype(Bc)::value;

@@ -1287,8 +1287,10 @@ struct Vecs {
   Scratch& sc;
   cudaStream_t s;
   std::vector<void*> extra;
-  ~Vecs() {
+  ~Vecs() { drop(); }
+  void drop() {
     for (void* p : extra) cudaFreeAsync(p, s);
+    extra.clear();
   }
   template <class T>
   T* get(long long n) {
@@ -1393,7 +1395,21 @@ int solve_device(SellMatrix& m, Scratch& sc, const SolveParams& p, const double*
   Plan plan;
   auto t0 = std::chrono::steady_clock::now();
 
-  const bool one_kernel = persist_applies(m, p);
+  bool one_kernel = persist_applies(m, p);
+  if (one_kernel) {
+    void* work = p.refuse == 2 ? nullptr : vec.get<char>((long long)persist_work_bytes(m, p));
+    rc = work ? persist_solve(m, p, d_b, d_x, work, sc.st, sc.hist, s) : kRefused;
+    if (rc == kRefused) {
+      // no room for its work vectors, or for a cooperative launch (an SM or
+      // block quota of this process): nothing has run; the kernels per phase
+      // need neither
+      cudaGetLastError();
+      vec.drop();
+      one_kernel = false;
+      rc = kOk;
+    }
+    if (rc) return rc;
+  }
   if (!one_kernel) rc = dispatch_ndof(nd, [&](auto Bc) -> int {
    constexpr int B = decltype(Bc)::value;
    return dispatch_u(p.precision == 0 ? m.u64 : m.u32, [&](auto Uc) -> int {
@@ -1949,10 +1965,6 @@ int solve_device(SellMatrix& m, Scratch& sc, const SolveParams& p, const double*
   };
 
   if (one_kernel) {
-    void* work = vec.get<char>((long long)persist_work_bytes(m, p));
-    if (!work) return kCudaError;
-    rc = persist_solve(m, p, d_b, d_x, work, sc.st, sc.hist, s);
-    if (rc) return rc;
     SolverState fin{};
     const cudaError_t e = read_state(fin);
     if (e != cudaSuccess) return report_cuda(e, "one-kernel solve", __FILE__, __LINE__);

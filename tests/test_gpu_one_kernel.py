@@ -209,3 +209,29 @@ def test_one_kernel_rule(gpu, dims, ndof, method, precision, one):
     m.device_prepare()
     rc, x, it = device_solve(m, b, False)
     assert rc == 1 and it == 3 and (m.Iarray[api.B200_PRM_I_LAUNCHES] == 1) == one
+
+
+@pytest.mark.parametrize("refuse", [1, 2])
+@pytest.mark.parametrize("method,precision", [(api.ITER_CG, 0), (api.ITER_CG, 1), (api.ITER_BICGSTAB, 0)])
+def test_one_kernel_refused_by_the_device(gpu, method, precision, refuse):
+    """A launch or an allocation of the one kernel that the device refuses (a
+    fake of the failing call): the same solve with a kernel per phase."""
+    index, item, val, b = grid_system((14, 11, 13), 2, 8)
+    n = len(index) - 1
+    m = api.Monolis(gpu)
+    m.set_matrix_BCSR(n, n, 2, len(item), val.reshape(-1), index, item)
+    m.quiet()
+    m.set_error_abort(False)
+    m.set_method(method)
+    m.set_precision(precision)
+    m.set_tolerance(1e-8)
+    m.device_prepare()
+    plain = device_solve(m, b, False)
+    assert plain[0] == 0 and m.Iarray[api.B200_PRM_I_LAUNCHES] == 1
+    m.Iarray[api.B200_PRM_I_REFUSE_LAUNCH] = refuse
+    rc, x, it = device_solve(m, b, False)
+    assert rc == 0 and m.Iarray[api.B200_PRM_I_LAUNCHES] > 1
+    if precision == 0:
+        assert it == plain[2] and bits_equal(x, plain[1])
+    else:
+        assert abs(it - plain[2]) <= 2 and np.linalg.norm(x - plain[1]) <= 1e-6 * np.linalg.norm(x)
