@@ -1259,7 +1259,7 @@ int monolis_b200_device_set_Dirichlet_bc_R(MONOLIS* m, double* d_b, int n_bc, co
   DevState* s = state_of(m);
   int rc = prepare(m, s, false, false, nullptr);
   if (rc) return rc;
-  rc = mb::device_dirichlet(s->A, d_b, n_bc, node_id, n_dof_bc, val, ctx().stream);
+  rc = mb::device_dirichlet(s->A, m->mat.NP, d_b, n_bc, node_id, n_dof_bc, val, ctx().stream);
   if (rc) return rc;
   return after_device_assembly(m, s);
 }

@@ -181,3 +181,35 @@ def test_refused_calls_change_nothing(gpu, ndof):
     for node, v in ((10, 1.5), (74, -2.0), (11, 0.5)):
         mh.set_Dirichlet_bc(b, node, 0, v)
     assert bits_equal(device_values(m, gpu), mh.values()) and bits_equal(d_b.cpu().numpy(), b)
+
+
+@pytest.mark.parametrize("ndof", [1, 3])
+def test_conditions_with_ghost_columns(gpu, ndof):
+    """One rank's part of a matrix: columns beyond its rows (ghosts) are never fixed by conditions on its own nodes."""
+    import torch
+    n, npn, rng = 40, 64, np.random.default_rng(13)
+    cols = [sorted({i, max(i - 1, 0), min(i + 1, n - 1), n + (7 * i) % (npn - n), npn - 1}) for i in range(n)]
+    index = np.concatenate([[0], np.cumsum([len(c) for c in cols])]).astype(np.int32)
+    item = np.concatenate(cols).astype(np.int32)
+    rows = np.repeat(np.arange(n), np.diff(index))
+    val = rng.standard_normal((len(item), ndof, ndof))
+    b = rng.standard_normal(n * ndof)
+    m = api.Monolis(gpu)
+    m.set_matrix_BCSR(n, npn, ndof, len(item), val.reshape(-1), index, item)
+    m.quiet()
+    nodes, dofs, vals = np.array([3, 39, 4], dtype=np.int32), np.array([0, ndof - 1, 0], dtype=np.int32), rng.standard_normal(3)
+    d_b = torch.from_numpy(b).cuda()
+    torch.cuda.synchronize()
+    assert gpu.monolis_b200_device_set_Dirichlet_bc_R(m.p, d_b.data_ptr(), 3, nodes.ctypes.data_as(api._ip),
+                                                      dofs.ctypes.data_as(api._ip), vals.ctypes.data_as(api._dp)) == 0
+    want, wb = val.copy(), b.reshape(n, ndof).copy()
+    for node, dof, v in zip(nodes, dofs, vals):  # one after the other, as the host call does
+        for k in np.flatnonzero(item == node):
+            wb[rows[k]] -= v * want[k, :, dof]
+            want[k, :, dof] = 0.0
+        want[rows == node, dof, :] = 0.0
+        want[(rows == node) & (item == node), dof, dof] = 1.0
+        wb[node, dof] = v
+    got = np.empty(len(item) * ndof * ndof)
+    assert gpu.monolis_b200_device_get_values(m.p, got.ctypes.data_as(api._dp)) == 0
+    assert bits_equal(got, want.reshape(-1)) and bits_equal(d_b.cpu().numpy(), wb.reshape(-1))
