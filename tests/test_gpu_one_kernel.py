@@ -17,14 +17,23 @@ from helpers import bits_equal
 pytestmark = pytest.mark.gpu
 
 
-def grid_system(dims, ndof, seed, shuffle=False, skew=0.0):
-    """7-point stencil on a grid of dims points with ndof x ndof blocks,
+def grid_system(dims, ndof, seed, shuffle=False, skew=0.0, points=7):
+    """7- or 27-point stencil on a grid of dims points with ndof x ndof blocks,
     diagonally dominant; skew != 0: nonsymmetric; shuffle: random numbering."""
     nx, ny, nz = dims
-    n = nx * ny * nz
-    rng = np.random.default_rng(seed)
-    ids = np.arange(n).reshape(nz, ny, nx)
+    ids = np.arange(nx * ny * nz).reshape(nz, ny, nx)
     pairs = [(ids[:, :, :-1], ids[:, :, 1:]), (ids[:, :-1], ids[:, 1:]), (ids[:-1], ids[1:])]
+    if points == 27:
+        def part(d, m):
+            return slice(max(0, -d), m - max(0, d)), slice(max(0, d), m + min(0, d))
+        offsets = [(0, 0, 1), (0, 1, -1), (0, 1, 0), (0, 1, 1)] + [(1, y, x) for y in (-1, 0, 1) for x in (-1, 0, 1)]
+        pairs = [[ids[q] for q in zip(*[part(d, m) for d, m in zip(o, (nz, ny, nx))])] for o in offsets]
+    return blocks_on(nx * ny * nz, pairs, ndof, seed, shuffle, skew)
+
+
+def blocks_on(n, pairs, ndof, seed, shuffle=False, skew=0.0, shift=0.05):
+    """The matrix of grid_system on n nodes that are coupled in pairs."""
+    rng = np.random.default_rng(seed)
     i = np.concatenate([np.arange(n)] + [a.ravel() for a, _ in pairs] + [b.ravel() for _, b in pairs])
     j = np.concatenate([np.arange(n)] + [b.ravel() for _, b in pairs] + [a.ravel() for a, _ in pairs])
     m = (len(i) - n) // 2
@@ -35,7 +44,7 @@ def grid_system(dims, ndof, seed, shuffle=False, skew=0.0):
         val[n + m:, r, r] = w * (1 + 0.1 * r) * (1 - skew)
     coupling = 0.1 * rng.standard_normal((ndof, ndof))
     val[:n] = coupling + coupling.T
-    diag = 0.05 + np.bincount(i[n:], weights=np.abs(val[n:]).sum(axis=2).max(axis=1), minlength=n) + 0.5 * ndof
+    diag = shift + np.bincount(i[n:], weights=np.abs(val[n:]).sum(axis=2).max(axis=1), minlength=n) + 0.5 * ndof
     val[np.arange(n), :, :] += diag[:, None, None] * np.eye(ndof)
     if shuffle:
         perm = rng.permutation(n)
@@ -43,6 +52,12 @@ def grid_system(dims, ndof, seed, shuffle=False, skew=0.0):
     order = np.lexsort((j, i))
     index = np.concatenate([[0], np.cumsum(np.bincount(i, minlength=n))]).astype(np.int32)
     return index, j[order].astype(np.int32), np.ascontiguousarray(val[order]), rng.uniform(0.0, 1.0, n * ndof)
+
+
+def residual(index, item, val, b, x):
+    ndof = val.shape[1]
+    ax = np.add.reduceat(np.einsum("krc,kc->kr", val, x.reshape(-1, ndof)[item]), index[:-1], axis=0)
+    return np.linalg.norm(b - ax.reshape(-1)) / np.linalg.norm(b)
 
 
 def device_solve(m, b, timers, offset=0):
@@ -82,7 +97,7 @@ def test_one_kernel_matches_kernels_per_phase(gpu, dims, ndof, shuffle, method, 
     rc0, x0, it0 = device_solve(m, b, True)
     for offset in (0, 1):  # x on a 16-byte boundary, and not
         rc1, x1, it1 = device_solve(m, b, False, offset)
-        assert rc1 == rc0
+        assert rc1 == rc0 and m.Iarray[api.B200_PRM_I_LAUNCHES] == 1
         if rc0:  # one row: BiCGSTAB divides by the exact zero residual on either path
             assert n == 1
             continue
@@ -90,10 +105,7 @@ def test_one_kernel_matches_kernels_per_phase(gpu, dims, ndof, shuffle, method, 
             assert it1 == it0 and bits_equal(x1, x0)
         else:
             assert abs(it1 - it0) <= 2, (it0, it1)
-            rows = np.repeat(np.arange(n), np.diff(index))
-            ax = np.zeros((n, ndof))
-            np.add.at(ax, rows, np.einsum("krc,kc->kr", val, x1.reshape(n, ndof)[item]))
-            assert np.linalg.norm(b - ax.reshape(-1)) / np.linalg.norm(b) < 1.01e-8
+            assert residual(index, item, val, b, x1) < 1.01e-8
 
 
 def test_one_kernel_initial_guess_log_and_limits(gpu):
@@ -235,3 +247,97 @@ def test_one_kernel_refused_by_the_device(gpu, method, precision, refuse):
         assert it == plain[2] and bits_equal(x, plain[1])
     else:
         assert abs(it - plain[2]) <= 2 and np.linalg.norm(x - plain[1]) <= 1e-6 * np.linalg.norm(x)
+
+
+def arrow(ndof, seed):
+    """9472 nodes in a ring, the first 64 coupled to 1500 nodes each besides:
+    two slices with most of the matrix, the rest short."""
+    n, hubs = 9472, 64
+    ring = np.arange(n)
+    far = np.arange(200, 200 + 6 * 1500, 6)
+    pairs = [(ring[:-1], ring[1:]), (np.repeat(np.arange(hubs), len(far)), np.tile(far, hubs))]
+    return blocks_on(n, pairs, ndof, seed, shift=5.0)
+
+
+# what the small grids do not reach: own vectors beyond the shared memory
+# (spill), matrix slices read from global memory, alone or beside cached ones,
+# slices with 32-bit column ids (a slot spans more than 65,535 columns), refined
+# CG without a window at ndof 1 to 3, and column bases beyond the room for them
+BOTH, ALL = [(api.ITER_CG, 0), (api.ITER_CG, 1)], [(api.ITER_CG, 0), (api.ITER_CG, 1), (api.ITER_BICGSTAB, 0)]
+
+
+@pytest.mark.parametrize("make,kw,ndof,method,precision", [
+    (make, kw, ndof, me, pr) for make, kw, ndof, which in [
+        (grid_system, dict(dims=(80, 80, 80)), 1, [(api.ITER_CG, 0)]),  # spill, all slices streamed
+        (grid_system, dict(dims=(96, 96, 100)), 1, [(api.ITER_CG, 1)]),
+        (grid_system, dict(dims=(61, 60, 59)), 1, ALL),
+        (grid_system, dict(dims=(44, 44, 40), shuffle=True), 1, ALL),  # 32-bit column ids, cached
+        (grid_system, dict(dims=(70, 70, 70), shuffle=True), 1, BOTH),  # and streamed
+        (grid_system, dict(dims=(64, 64, 62), shuffle=True), 1, [(api.ITER_BICGSTAB, 0)]),
+        (grid_system, dict(dims=(31, 31, 32), shuffle=True), 2, ALL),
+        (grid_system, dict(dims=(27, 27, 28), shuffle=True), 3, BOTH),
+        (grid_system, dict(dims=(31, 32, 31), points=27), 3, ALL),  # cached and streamed slices in a block
+        (grid_system, dict(dims=(60, 60, 30), points=27), 3, BOTH),  # window, spill, streamed
+        (grid_system, dict(dims=(30, 31, 29)), 6, BOTH),
+        (arrow, {}, 1, ALL), (arrow, {}, 3, BOTH),
+    ] for me, pr in which])
+def test_one_kernel_large(gpu, make, kw, ndof, method, precision):
+    if method == api.ITER_BICGSTAB and make is grid_system:
+        kw = dict(kw, skew=0.3)
+    index, item, val, b = make(ndof=ndof, seed=4, **kw)
+    n = len(index) - 1
+    m = api.Monolis(gpu)
+    m.set_matrix_BCSR(n, n, ndof, len(item), val.reshape(-1), index, item)
+    m.quiet()
+    m.set_error_abort(False)
+    m.set_method(method)
+    m.set_precision(precision)
+    m.set_tolerance(1e-8)
+    m.set_maxiter(500)
+    m.Iarray[api.B200_PRM_I_ITER_RR] = 7
+    m.device_prepare()
+    rc0, x0, it0 = device_solve(m, b, True)
+    rc1, x1, it1 = device_solve(m, b, False)
+    assert m.Iarray[api.B200_PRM_I_LAUNCHES] == 1
+    assert rc1 == rc0 == 0
+    wide = m.Iarray[api.B200_PRM_I_WIDE_SLICES_FP32 if precision else api.B200_PRM_I_WIDE_SLICES_FP64]
+    if ndof == 1 and kw.get("shuffle"):
+        assert wide > 0
+    if precision == 0:
+        assert it1 == it0 and bits_equal(x1, x0)
+    else:
+        assert abs(it1 - it0) <= 2 and residual(index, item, val, b, x1) < 1.01e-8
+
+
+@pytest.mark.parametrize("method,precision", ALL)
+def test_one_kernel_odd_values(gpu, method, precision):
+    """Rows without entries (whole slices of them in either layout), and right-hand
+    sides with Inf, NaN, squares that overflow or vanish: the status and the count
+    of the kernels per phase."""
+    index, item, val, b = grid_system((16, 15, 14), 1, 6, skew=0.3 if method == api.ITER_BICGSTAB else 0.0)
+    n = len(index) - 1
+    rows = np.repeat(np.arange(n), np.diff(index))
+    gone = lambda k: (k >= 64) & (k < 200)
+    keep = ~gone(rows) & ~gone(item)
+    index2 = np.concatenate([[0], np.cumsum(np.bincount(rows[keep], minlength=n))]).astype(np.int32)
+    rhs = [(index2, item[keep], val[keep], b)]
+    for k, v in ((3, np.inf), (700, np.nan), (9, 1e200)):
+        c = b.copy()
+        c[k] = v
+        rhs.append((index, item, val, c))
+    rhs.append((index, item, val, b * 1e-200))
+    for index_, item_, val_, b_ in rhs:
+        m = api.Monolis(gpu)
+        m.set_matrix_BCSR(n, n, 1, len(item_), val_.reshape(-1), index_, item_)
+        m.quiet()
+        m.set_error_abort(False)
+        m.set_method(method)
+        m.set_precision(precision)
+        m.set_tolerance(1e-8)
+        m.set_maxiter(6)
+        m.device_prepare()
+        rc0, x0, it0 = device_solve(m, b_, True)
+        rc1, x1, it1 = device_solve(m, b_, False)
+        assert rc1 == rc0 and it1 == it0
+        if precision == 0 and np.isfinite(x0).all():
+            assert bits_equal(x1, x0)
