@@ -32,10 +32,8 @@ __device__ __forceinline__ float sub_rn(float a, float b) { return a - b; }
 __device__ __forceinline__ double axpy_rn(double a, double x, double y) { return __dadd_rn(__dmul_rn(a, x), y); }
 __device__ __forceinline__ float axpy_rn(float a, float x, float y) { return fmaf(a, x, y); }
 
-// ---- streaming loads: matrix values and column ids are read once per SpMV,
-// so they are loaded with the evict-first hint to keep x resident in L1/L2.
-__device__ __forceinline__ double ld_stream(const double* p) { return __ldcs(p); }
-__device__ __forceinline__ float ld_stream(const float* p) { return __ldcs(p); }
+// ---- streaming loads: column ids are read once per SpMV, so they are loaded
+// with the evict-first hint to keep x resident in L1/L2 (values: spmv.cuh).
 __device__ __forceinline__ int ld_stream(const int* p) { return __ldcs(p); }
 __device__ __forceinline__ short ld_stream(const short* p) { return __ldcs(p); }
 

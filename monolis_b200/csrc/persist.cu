@@ -14,8 +14,11 @@
 // they fit.
 //
 // Arithmetic is that of solve.cu, expression by expression: FP64 row sums in
-// CSR order, two roundings per a*b + c, dot products in double-double (the
-// grouping of the partial sums differs, their value does not: common.cuh).
+// CSR order, two roundings per a*b + c, dot products in double-double. The
+// partial sums are grouped otherwise and renormalised less often, so a dot
+// product rounds to the same bits unless its exact value lies within a few n
+// eps^2 sum |x_i y_i| of a rounding boundary; every solve compared had the bits
+// of the kernels per phase.
 #include <algorithm>
 #include <cstdio>
 
@@ -57,9 +60,10 @@ __device__ __forceinline__ void fence_gpu() { asm volatile("fence.acq_rel.gpu;" 
 
 // (hi, lo) += (h2, l2) without renormalising: the error of the leading sum is
 // exact (TwoSum) and the low parts are added in double, so a tree of a few
-// levels keeps |lo| within a few ulps of hi and loses a few eps^2 of it; its
-// chain is one addition a level where dd_merge's is ten, which is what a
-// reduction over lanes waits for.
+// levels loses a few eps^2 of the sum of the absolute partial sums (under
+// cancellation that is more of the result than dd_merge loses); its chain is
+// one addition a level where dd_merge's is ten, which is what a reduction over
+// lanes waits for.
 __device__ __forceinline__ void dd_merge_raw(double& hi, double& lo, double h2, double l2) {
   double s, e;
   two_sum(hi, h2, s, e);
@@ -652,12 +656,12 @@ struct SumXY {
 };
 
 // r = b - A x (refined: b - A (x + y), stored FP32) on the block's rows, and
-// CG: z = M^-1 r, sums <r,r>, <r,z>; BiCGSTAB: <r,r>, <r,rt> (rt = r first).
+// CG: z = M^-1 r, sums <r,r>, <r,z>; BiCGSTAB: <r,r>, <r,rt> (init: rt = r).
 // Sums in double-double in either precision, as in the kernels per phase: the
 // residual that decides convergence does not depend on their grouping.
 template <int B, class T, bool Bicg>
-__device__ __forceinline__ void residual(const PersistArgs<T>& a, const BlockRows<T>& m, T* r, T* rt /* CG: z */, bool init,
-                                         DDAcc<2>& v) {
+__device__ __forceinline__ void residual(const PersistArgs<T>& a, const BlockRows<T>& m, T* r, T* rt /* CG: z */,
+                                         DDAcc<2>& v, bool init = false) {
   constexpr bool kMixed = sizeof(T) == 4;
   constexpr int UR = B == 1 ? 4 : (B <= 3 ? 2 : 1);
   for (int row = m.r0 + (int)threadIdx.x; row < m.r1; row += blockDim.x) {
@@ -747,7 +751,7 @@ __global__ void __launch_bounds__(TH, 1) persist_cg_kernel(const PersistArgs<T> 
   Pipe<B, U, D, T> pipe;
   {
     DDAcc<2> v;
-    residual<B, T, false>(a, m, r, z, true, v);
+    residual<B, T, false>(a, m, r, z, v);
     fill_pipe(a, m, pipe);
     if (!grid_exchange(ex, sh, v, finish)) return;
   }
@@ -838,7 +842,7 @@ __global__ void __launch_bounds__(TH, 1) persist_cg_kernel(const PersistArgs<T> 
       copy_own<B, T>(m, xg, xo);
       if (!grid_barrier(ex, sh)) return;
       DDAcc<2> w;
-      residual<B, T, false>(a, m, r, z, false, w);
+      residual<B, T, false>(a, m, r, z, w);
       if (!grid_exchange(ex, sh, w, finish)) return;
     }
   }
@@ -878,7 +882,7 @@ __global__ void __launch_bounds__(TH, 1) persist_bicg_kernel(const PersistArgs<d
   Pipe<B, U, D, T> pipe;
   {
     DDAcc<2> v;
-    residual<B, T, true>(a, m, r, rt, true, v);
+    residual<B, T, true>(a, m, r, rt, v, true);
     if (!grid_exchange(ex, sh, v, finish)) return;
   }
   const bool alu_vec = (a.N % group_rows<B, T>()) == 0;
@@ -1008,7 +1012,7 @@ __global__ void __launch_bounds__(TH, 1) persist_bicg_kernel(const PersistArgs<d
       copy_own<B, T>(m, a.x, xo);
       if (!grid_barrier(ex, sh)) return;
       DDAcc<2> w;
-      residual<B, T, true>(a, m, r, rt, false, w);
+      residual<B, T, true>(a, m, r, rt, w);
       if (!grid_exchange(ex, sh, w, finish)) return;
     }
   }

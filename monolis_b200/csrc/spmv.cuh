@@ -205,7 +205,7 @@ __device__ __forceinline__ void load_cols2(bool wide, bool uniform, const int2* 
 // longer length.
 // The entries of the multiplied vector come from xf(i) (i = column*B + l):
 // a plain gather, or a value computed from other vectors (see sell_row2).
-template <int B, int U, bool kCols16 = true, int P = kStreamOnce, class XF>
+template <int B, int U, bool kCols16 = true, class XF>
 __device__ __forceinline__ void sell_row2_f(const SellView2& A, const XF xf, int t, float (&y0)[B], float (&y1)[B]) {
   constexpr int B2 = B * B;
   const int r0 = 2 * t;
@@ -231,7 +231,7 @@ __device__ __forceinline__ void sell_row2_f(const SellView2& A, const XF xf, int
 #pragma unroll
     for (int u = 0; u < U; u++)
 #pragma unroll
-      for (int e = 0; e < B2; e++) a[u][e] = ld_mat<P>(v + ((long long)(k + u) * B2 + e) * 32);
+      for (int e = 0; e < B2; e++) a[u][e] = ld_stream2(v + ((long long)(k + u) * B2 + e) * 32);
 #pragma unroll
     for (int u = 0; u < U; u++) {
       float x0[B], x1[B];
@@ -259,7 +259,7 @@ __device__ __forceinline__ void sell_row2_f(const SellView2& A, const XF xf, int
     for (int u = 0; u < U; u++)
 #pragma unroll
       for (int e = 0; e < B2; e++)
-        a[u][e] = u < rem ? ld_mat<P>(v + ((long long)(k + u) * B2 + e) * 32) : make_float2(0.f, 0.f);
+        a[u][e] = u < rem ? ld_stream2(v + ((long long)(k + u) * B2 + e) * 32) : make_float2(0.f, 0.f);
     float x0[U][B], x1[U][B];
 #pragma unroll
     for (int u = 0; u < U; u++)
