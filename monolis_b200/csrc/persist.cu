@@ -126,8 +126,12 @@ struct AccWords<DDAcc<K>> {
 // threads have met at a block barrier) is visible to every block that passes.
 __device__ __forceinline__ bool arrive_and_wait(Exchange& x) {
   unsigned long long v, n = 0;
-  if (x.target == x.delay_at && blockIdx.x == 0)
+  // (compared whole, the words cost up to 1 us an iteration, by the code laid
+  // out around them: 8^3 refined 11.8 against 10.7)
+  if ((unsigned int)x.target == (unsigned int)x.delay_at && blockIdx.x == 0) {
+#pragma unroll 1
     for (unsigned int t = 0; t < x.delay_ns; t += 1000) __nanosleep(1000);
+  }
   fence_gpu();
   asm volatile("red.relaxed.gpu.global.add.u64 [%0], 1;" ::"l"(&x.slots->arrived) : "memory");
   bool ok = true;
@@ -1022,10 +1026,12 @@ __global__ void __launch_bounds__(TH, 1) persist_bicg_kernel(const PersistArgs<d
 }
 
 // Threads of a block, slots of a chunk and chunk buffers, by block size.
-template <int B, class T>
+// BiCGSTAB at 3x3 has no registers for three slots: 28^3 nodes 46 us an
+// iteration (41 where the compiler happens to spill), two slots 40.
+template <int B, class T, bool Bicg>
 struct Shape {
   static constexpr int threads = B == 1 ? 512 : 256;
-  static constexpr int u = B == 1 ? 4 : (B <= 3 ? 3 : 1);
+  static constexpr int u = B == 1 ? 4 : (B <= 3 ? (Bicg && B == 3 ? 2 : 3) : 1);
   static constexpr int d = B == 1 ? 3 : 2;
 };
 constexpr int kSmemBytes = 220 * 1024, kSmemCache = 180 * 1024;
@@ -1174,10 +1180,11 @@ int persist_solve(const SellMatrix& m, const SolveParams& p, const double* b, do
     constexpr int B = decltype(Bc)::value;
     auto pick = [&](auto Wc, auto a) -> int {
       using T = std::remove_pointer_t<decltype(a.z)>;
-      using Sh = Shape<B, T>;
+      using Sh = Shape<B, T, false>;
+      using Sb = Shape<B, T, true>;
       constexpr bool W = decltype(Wc)::value && B <= kWindowMaxNdof;
       if (p.method == 1) return run(persist_cg_kernel<B, Sh::u, Sh::d, Sh::threads, W, T>, a, Sh::threads);
-      if constexpr (sizeof(T) == 8) return run(persist_bicg_kernel<B, Sh::u, Sh::d, Sh::threads>, a, Sh::threads);
+      if constexpr (sizeof(T) == 8) return run(persist_bicg_kernel<B, Sb::u, Sb::d, Sb::threads>, a, Sb::threads);
       else return kBadInput;
     };
     if (p.precision == 0)
