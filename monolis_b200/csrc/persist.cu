@@ -1096,16 +1096,17 @@ size_t persist_work_bytes(const SellMatrix& m, const SolveParams& p) {
 // of 200 to 400 iterations; the stream in MB, 7- or 27-entry rows, grids in natural
 // and in random numbering and plates too wide for the window):
 //   CG, FP64      ndof 1  0.1 MB 30 / 8.8, 24 MB 28 / 16, no window: 47 MB 40 / 32, 50 MB 32 / 29
-//                 ndof 2  49 MB 39 / 27, 61 MB 36 / 33, 77 MB 39 / 39, 87 MB 42 / 44
+//                 ndof 2  49 MB 39 / 27, 66 MB 38 / 35, 76 MB 41 / 39, 87 MB 41 / 45
 //                 ndof 3  0.8 MB 31 / 12, 134 MB 42 / 34, 218 MB 67 / 52, 245 MB 66 / 62; no window: 93 MB 46 / 33
-//                 ndof 4  93 MB 39 / 34;   ndof 5  94 MB 40 / 30;   ndof 6  82 MB 40 / 35, 90 MB 40 / 40
+//                 ndof 4  93 MB 39 / 34;   ndof 5  94 MB 40 / 30;   ndof 6  82 MB 40 / 35, 97 MB 42 / 40
 //   CG, refined   ndof 1  7 MB 24 / 8.5, 50 MB 31 / 24; no window: 48 MB 46 / 37, 60 MB 35 / 34
-//                 ndof 2  56 MB 35 / 30, 79 MB 40 / 37, 84 MB 40 / 43
+//                 ndof 2  56 MB 35 / 30, 79 MB 40 / 37, 87 MB 42 / 41, 110 MB 48 / 49
 //                 ndof 3  8 MB 28 / 11, 127 MB 42 / 36, 210 MB 60 / 51, 244 MB 66 / 67
 //                 ndof 4  91 MB 39 / 36;   ndof 5  93 MB 40 / 29;   ndof 6  91 MB 42 / 37
 //   BiCGSTAB      ndof 1  1.2 MB 47 / 20, 31 MB 49 / 40, 60 MB 69 / 82
-//                 ndof 2  47 MB 55 / 50, 61 MB 59 / 64;   ndof 3  63 MB 62 / 53, 76 MB 64 / 72 (random numbering 72 / 91)
-//                 ndof 4  93 MB 68 / 66;   ndof 5  94 MB 70 / 66;   ndof 6  82 MB 69 / 64, 90 MB 69 / 74
+//                 ndof 2  47 MB 55 / 50, 57 MB 56 / 57, 63 MB 61 / 64
+//                 ndof 3  70 MB 63 / 46, 76 MB 64 / 62 (random numbering 73 / 82), 83 MB 67 / 70
+//                 ndof 4  107 MB 72 / 69;   ndof 5  101 MB 71 / 63;   ndof 6  84 MB 67 / 63, 89 MB 69 / 71
 // Refined BiCGSTAB stays with the kernels per phase: its dot products cancel,
 // so its FP32 recurrences hang on the grouping of their plain sums (symmetric
 // elasticity, 33^3 nodes: 1467 iterations with one, none within 20000 with
@@ -1118,8 +1119,8 @@ bool persist_applies(const SellMatrix& m, const SolveParams& p) {
   if (p.shard || p.np_rows != m.N || p.timers || (p.method != 1 && (p.method != 5 || mixed))) return false;
   const PersistPlan q = make_plan(m, p);
   // MB by ndof; ndof 3 without a window: 100
-  static constexpr double kCg[6] = {50, 70, 250, 100, 100, 90}, kCgMixed[6] = {60, 80, 225, 100, 100, 100},
-                          kBicg[6] = {32, 52, 65, 95, 95, 80};
+  static constexpr double kCg[6] = {50, 75, 250, 100, 100, 100}, kCgMixed[6] = {60, 88, 225, 100, 100, 100},
+                          kBicg[6] = {32, 54, 74, 100, 100, 86};
   double limit = (p.method == 5 ? kBicg : mixed ? kCgMixed : kCg)[m.ndof - 1];
   if (p.method == 1 && !q.window) limit = std::min(limit, 100.0);
   return q.ok && (mixed ? m.bytes32 : m.bytes64) <= limit * 1e6;

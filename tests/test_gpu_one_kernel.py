@@ -202,10 +202,11 @@ def test_one_kernel_any_wait_runs_out(gpu, ndof, shuffle, method, precision):
 
 
 @pytest.mark.parametrize("dims,ndof,method,precision,one", [
-    ((58, 58, 58), 2, api.ITER_CG, 0, True), ((66, 66, 66), 2, api.ITER_CG, 0, False),  # 52 and 76 MB
-    ((132, 132, 36), 2, api.ITER_CG, 1, False),  # 87 MB
-    ((55, 55, 55), 2, api.ITER_BICGSTAB, 0, True), ((62, 62, 62), 2, api.ITER_BICGSTAB, 0, False),  # 44 and 63 MB
-    ((52, 52, 52), 3, api.ITER_BICGSTAB, 0, False), ((35, 35, 36), 6, api.ITER_BICGSTAB, 0, False),  # 78 and 92 MB
+    ((62, 62, 62), 2, api.ITER_CG, 0, True), ((67, 67, 67), 2, api.ITER_CG, 0, False),  # 63 and 80 MB
+    ((132, 132, 34), 2, api.ITER_CG, 1, True), ((132, 132, 38), 2, api.ITER_CG, 1, False),  # 82 and 92 MB
+    ((57, 57, 57), 2, api.ITER_BICGSTAB, 0, True), ((62, 62, 62), 2, api.ITER_BICGSTAB, 0, False),  # 49 and 63 MB
+    ((50, 50, 50), 3, api.ITER_BICGSTAB, 0, True), ((52, 52, 52), 3, api.ITER_BICGSTAB, 0, False),  # 70 and 78 MB
+    ((35, 35, 36), 6, api.ITER_BICGSTAB, 0, False),  # 92 MB
 ])
 def test_one_kernel_rule(gpu, dims, ndof, method, precision, one):
     """One kernel up to the matrix stream at which the kernels per phase take over, by method and block size."""
