@@ -44,12 +44,12 @@ constexpr unsigned long long kSpinLimit = 1ull << 22;
 // an SM, so that an SM's rows are one run and the barrier has few arrivals; the
 // threads are what the registers allow without spilling much. 1x1: 768 of 80
 // registers, or in FP32, where an iteration's vectors do not stay in L2
-// (kStride), 1024 of 64 (more loads in flight for HBM). 2x2: 768 in FP32, 512
-// in FP64 (768 spill 800 bytes: 52^3 x 32 right-hand sides, 7-entry rows, 278
-// us an iteration against 230; 20^3 x 5 32.9 and 29.1). Larger blocks run as
-// many blocks of 256 as fit; the blocks loaded ahead spill 1.1 KB at 6x6 in
-// FP64 and 110 bytes at 5x5 (40^3 x 5: ndof 6 260 us an iteration with them,
-// 210 without; ndof 5 166 and 151) and are left out there.
+// (kStride), 1024 of 64 (more loads in flight for HBM: 96^3 x 32 right-hand
+// sides, 7-entry rows, 417 us an iteration, 768 threads 492). 2x2: 768 in FP32,
+// 512 in FP64 (768 spill 800 bytes: 52^3 x 32 256 us against 207, 20^3 x 5 29.4
+// and 26.0). Larger blocks run as many blocks of 256 as fit; the blocks loaded
+// ahead spill 1.1 KB at 6x6 in FP64 and 110 bytes at 5x5 (40^3 x 32: ndof 6 472
+// us with them, 429 without; ndof 5 367 and 319) and are left out there.
 template <int B, class T, bool kStride>
 struct MultiShape {
   static constexpr bool fp32 = sizeof(T) == 4;
