@@ -465,7 +465,7 @@ int device_add_elements(SellMatrix& m, int NP, int n_elem, int n_base, const int
 int device_dirichlet(SellMatrix& m, int NP, double* d_b, int n_bc, const int* node, const int* dof, const double* val,
                      cudaStream_t s) {
   const int N = m.N, nd = m.ndof;
-  const long long n = (long long)NP * nd;  // columns: ghosts, never fixed here, after the own rows
+  const long long n = (long long)std::max(N, NP) * nd;  // columns: ghosts, never fixed here, after the own rows
   std::vector<long long> flat((size_t)n_bc);
   for (int q = 0; q < n_bc; q++) {
     if (node[q] < 0 || node[q] >= N || dof[q] < 0 || dof[q] >= nd) return kBadInput;
